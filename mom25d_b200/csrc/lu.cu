@@ -5,14 +5,13 @@
 // (fast.py:356-358). Pivots follow zgetrf: the largest |re| + |im| of the column (izamax), the first on ties.
 //
 // Per panel of nb columns:
-//   1. k_panel     cooperative kernel over all SMs: the panel's rows split between the blocks; per column one grid
-//                  barrier (bounded) after each block publishes its candidate pivot row, then every block applies
-//                  the interchange and the rank-1 update to its own rows.
+//   1. the panel   one thread-block cluster with the panel's columns in registers (panel.cu) where its rows fit;
+//                  else k_panel_smem, a cooperative kernel with the rows in shared memory, or k_panel with the rows in
+//                  global memory and a bounded grid barrier a column.
 //   2. k_laswp     the panel's interchanges applied to the columns left and right of it.
 //   3. k_trsm      U12 = L11^-1 A12 (unit lower), one thread per column, L11 in shared memory.
 //   4. trailing    A22 -= L21 U12: the complex SIMT GEMM below (FP64 / FP32), or the tensor-core 3xTF32 product
 //                  (umma.cu) for complex64 with tf32 on.
-#include <cooperative_groups.h>
 #include <type_traits>
 #include <algorithm>
 #include <mutex>
@@ -25,6 +24,9 @@ int m25_check_dev_err(cudaStream_t s, const char *what);
 int m25_umma_trailing(float *A, long lda, int M, int Ncol, int K, const float *L21, const float *U12, void *work,
                       size_t work_bytes, cudaStream_t s);
 size_t m25_umma_workspace(int n, int nb);
+int m25_panel_cluster_max(int single);
+int m25_panel_cluster_rows(int single, int cl);
+int m25_panel_cluster(void *A, long lda, int n, int k0, int jb, int *ipiv, int single, int cl, int *err, cudaStream_t s);
 
 #define NB 64
 #define NB2 256
@@ -78,54 +80,8 @@ __device__ __forceinline__ bool ll_wait(const unsigned long long *p, int stride,
 }
 
 
-// The same exchange inside a thread-block cluster: each block's records in its own shared memory, written there and
-// read by the other blocks of the cluster through distributed shared memory (generic addresses of their shared
-// memory), at cluster scope; polled the same bounded way.
-__device__ __forceinline__ void cl_put(unsigned long long *p, unsigned payload, unsigned flag)
-{
-    const unsigned long long w = ((unsigned long long)flag << 32) | payload;
-    asm volatile("st.relaxed.cluster.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
-}
-__device__ __forceinline__ unsigned long long cl_get(const unsigned long long *p)
-{
-    unsigned long long w;
-    asm volatile("ld.relaxed.cluster.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
-    return w;
-}
-template <bool CL>
-__device__ __forceinline__ void x_put(unsigned long long *p, unsigned payload, unsigned flag)
-{
-    if (CL) cl_put(p, payload, flag);
-    else ll_put(p, payload, flag);
-}
-template <int K, bool CL>
-__device__ __forceinline__ bool x_wait(const unsigned long long *p, int stride, unsigned flag, unsigned *out,
-                                       const int *err)
-{
-    if (!CL) return ll_wait<K>(p, stride, flag, out, err);
-    long it = 0;
-    for (;;) {
-        bool all = true;
-#pragma unroll
-        for (int q = 0; q < K; ++q) {
-            const unsigned long long w = cl_get(p + (size_t)q * stride);
-            out[q] = (unsigned)w;
-            all = all && (unsigned)(w >> 32) == flag;
-        }
-        if (all) return true;
-        if ((++it & 1023) == 0 && (it > (1L << 22) || *(volatile const int *)err)) return false;
-    }
-}
-
 #define PANEL_NONE 0x7fffffff
 #define LL_REC 32             // words a candidate record (256 bytes: polled by every block, one record a line pair)
-// a cluster panel's records, after its rows in shared memory
-struct PanelRecords {
-    unsigned long long cand[2][LL_REC];
-    unsigned long long row[2][4 * NB];
-    unsigned long long drow[2][4 * NB];
-};
-
 // The largest |re| + |im| and its row over a warp (the first row on ties: izamax / icamax)
 template <typename R>
 __device__ __forceinline__ void warp_argmax(R &v, int &row)
@@ -153,12 +109,6 @@ __device__ __forceinline__ void warp_argmax(R &v, int &row)
 // due on the columns past the group added on the way, not stored), the diagonal row as stored (it moves into
 // another block's rows, where those terms are still applied). Every entry still takes its terms a -= l U one at a
 // time in column order: the results are those of the column-by-column order.
-//
-// CL: the panel's blocks are one thread-block cluster (a panel of up to 16 blocks' rows) and the exchange goes
-// through distributed shared memory instead of L2: the same records and bounded polls, each block's records after
-// its rows in its own shared memory (zeroed, then a cluster barrier, before the first column; a cluster barrier
-// before any block leaves, so that no block reads the shared memory of one that has). The other blocks' records
-// are a few hundred cycles away instead of an L2 round trip, which the trailing update's traffic makes long.
 #define GRP 8
 // the block's candidate from the warps' ones (sv, si of nw warps): one butterfly in every warp
 template <typename R>
@@ -168,7 +118,7 @@ __device__ __forceinline__ void block_argmax(R &v, int &row, const R *sv, const 
     row = lane < nw ? si[lane] : PANEL_NONE;
     warp_argmax(v, row);
 }
-template <typename R, bool CL>
+template <typename R>
 __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, int n, int k0, int jb, int *ipiv,
                                                               PanelWork pw, int *err)
 {
@@ -185,7 +135,6 @@ __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, in
     const int r0 = k0 + b * cs, r1 = min(n, r0 + cs);
     const int nr = max(0, r1 - r0);
     const int PW = jb * WPC;                              // payload words of one panel row
-    PanelRecords *RX = reinterpret_cast<PanelRecords *>(panel_raw + ((size_t)cs * jb * sizeof(C) + 15) / 16 * 16);
     __shared__ __align__(16) C U[NB], D[NB], W[NB];       // pivot row, diagonal row, this block's published row
     __shared__ __align__(16) C Ug[GRP][NB];               // the current group's pivot rows
     __shared__ R sv[NWARP], sv2[NWARP];
@@ -196,12 +145,6 @@ __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, in
         Ps[c * cs + i] = ldc<R>(A, (size_t)(k0 + c) * lda + r0 + i);
     }
     if (tid == 0) s_fail = 0;
-    if constexpr (CL) {
-        unsigned long long *rz = reinterpret_cast<unsigned long long *>(RX);
-        for (int e = tid; e < (int)(sizeof(PanelRecords) / 8); e += PANEL_THREADS) rz[e] = 0ull;
-        __syncthreads();
-        cooperative_groups::this_cluster().sync();
-    }
     __syncthreads();
     R best = -1;                                          // this thread's candidate for column 0
     int bi = PANEL_NONE;
@@ -214,22 +157,12 @@ __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, in
         const unsigned flag = (unsigned)col + 1u;
         const bool own_col = col >= r0 && col < r1;
         // this column's records: where this block publishes, and where block q's are read
-        unsigned long long *my_rec, *my_row, *my_drow;
-        if constexpr (CL) {
-            my_rec = RX->cand[par]; my_row = RX->row[par]; my_drow = RX->drow[par];
-        } else {
-            my_rec = pw.ll_cand + ((size_t)par * G + b) * LL_REC;
-            my_row = pw.ll_row + ((size_t)par * G + b) * (4 * NB);
-            my_drow = pw.ll_drow + (size_t)par * (4 * NB);
-        }
+        unsigned long long *my_rec = pw.ll_cand + ((size_t)par * G + b) * LL_REC;
+        unsigned long long *my_row = pw.ll_row + ((size_t)par * G + b) * (4 * NB);
+        unsigned long long *my_drow = pw.ll_drow + (size_t)par * (4 * NB);
         auto rec_of = [&](int q, int which) -> const unsigned long long * {   // which: 0 record, 1 row, 2 diagonal
-            if constexpr (CL) {
-                unsigned long long *mine = which == 0 ? RX->cand[par] : which == 1 ? RX->row[par] : RX->drow[par];
-                return cooperative_groups::this_cluster().map_shared_rank(mine, (unsigned)q);
-            } else {
-                return which == 0 ? pw.ll_cand + ((size_t)par * G + q) * LL_REC
-                     : which == 1 ? pw.ll_row + ((size_t)par * G + q) * (4 * NB) : pw.ll_drow + (size_t)par * (4 * NB);
-            }
+            return which == 0 ? pw.ll_cand + ((size_t)par * G + q) * LL_REC
+                 : which == 1 ? pw.ll_row + ((size_t)par * G + q) * (4 * NB) : pw.ll_drow + (size_t)par * (4 * NB);
         };
         const int g0 = j - j % GRP, gend = min(g0 + GRP, jb);
         const bool gstart = j > 0 && j == g0;             // the previous group's terms are due past column j
@@ -273,8 +206,8 @@ __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, in
             if (lane == 0) {
                 const unsigned *bv32 = reinterpret_cast<const unsigned *>(&best);
 #pragma unroll
-                for (int q = 0; q < VW; ++q) x_put<CL>(rec + q, bv32[q], flag);
-                x_put<CL>(rec + VW, (unsigned)bi, flag);
+                for (int q = 0; q < VW; ++q) ll_put(rec + q, bv32[q], flag);
+                ll_put(rec + VW, (unsigned)bi, flag);
             }
             unsigned long long *rrow = my_row;
             unsigned long long *drow = my_drow;
@@ -286,13 +219,13 @@ __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, in
                     W[c] = a;
                     const unsigned *a32 = reinterpret_cast<const unsigned *>(&a);
 #pragma unroll
-                    for (int q = 0; q < WPC; ++q) x_put<CL>(rrow + c * WPC + q, a32[q], flag);
+                    for (int q = 0; q < WPC; ++q) ll_put(rrow + c * WPC + q, a32[q], flag);
                 }
                 if (own_col) {                             // the diagonal row as stored
                     const C d = Ps[c * cs + ec];
                     const unsigned *d32 = reinterpret_cast<const unsigned *>(&d);
 #pragma unroll
-                    for (int q = 0; q < WPC; ++q) x_put<CL>(drow + c * WPC + q, d32[q], flag);
+                    for (int q = 0; q < WPC; ++q) ll_put(drow + c * WPC + q, d32[q], flag);
                 }
             }
             __syncwarp();
@@ -333,7 +266,7 @@ __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, in
         int brow = PANEL_NONE, bw = -1;
         if (tid < G) {
             unsigned wv[VW + 1];
-            if (!x_wait<VW + 1, CL>(rec_of(tid, 0), 1, flag, wv, err)) {
+            if (!ll_wait<VW + 1>(rec_of(tid, 0), 1, flag, wv, err)) {
                 s_fail = 1;
                 dev_error(err, M25_DEV_TIMEOUT);
             } else if ((int)wv[VW] != PANEL_NONE) {
@@ -349,7 +282,7 @@ __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, in
         }
         if (lane == 0) { sv2[wid] = bv; si2[wid] = brow; sw2[wid] = bw; }
         __syncthreads();                                  // (and the deferred update is complete)
-        if (s_fail) goto finish;
+        if (s_fail) return;
         bv = lane < NWARP ? sv2[lane] : (R)-1;              // the block's reduction by one butterfly a warp
         brow = lane < NWARP ? si2[lane] : PANEL_NONE;
         bw = lane < NWARP ? sw2[lane] : -1;
@@ -360,7 +293,7 @@ __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, in
         }
         if (bw < 0 || bw >= G) {
             if (tid == 0) dev_error(err, M25_DEV_INDEX);
-            goto finish;
+            return;
         }
         const int p = brow;
         if (b == 0 && tid == 0) ipiv[col] = p;
@@ -375,9 +308,9 @@ __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, in
             if (own_p) {
                 u = reinterpret_cast<const unsigned *>(W)[tid];
                 if (own_col) d = P32[((size_t)(tid / WPC) * cs + (col - r0)) * WPC + q];
-                else ok = x_wait<1, CL>(rec_of((col - k0) / cs, 2) + tid, 0, flag, &d, err);
+                else ok = ll_wait<1>(rec_of((col - k0) / cs, 2) + tid, 0, flag, &d, err);
             } else if (need_u) {
-                ok = x_wait<1, CL>(rec_of(bw, 1) + tid, 0, flag, &u, err);
+                ok = ll_wait<1>(rec_of(bw, 1) + tid, 0, flag, &u, err);
             }
             if (!ok) {
                 s_fail = 1;
@@ -391,7 +324,7 @@ __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, in
             }
         }
         __syncthreads();
-        if (s_fail) goto finish;
+        if (s_fail) return;
         // (6) rows col and p interchanged (whole panel rows), column j scaled by 1 / pivot, column j + 1 updated
         // (the rest of this column's update is deferred to the next column's step 3); the next candidates
         const C piv = U[j];
@@ -436,8 +369,6 @@ __global__ void __launch_bounds__(PANEL_THREADS) k_panel_smem(R *A, long lda, in
         int c = e / nr, i = e % nr;
         stc<R>(A, (size_t)(k0 + c) * lda + r0 + i, Ps[c * cs + i]);
     }
-finish:
-    if constexpr (CL) cooperative_groups::this_cluster().sync();   // (no block leaves while another may read it)
 }
 
 // The same with the rows in global memory (when a block's rows do not fit in shared memory).
@@ -1839,37 +1770,17 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
     M25_CHECK(cudaGetDevice(&dev));
     M25_CHECK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     cudaFuncAttributes pfa;
-    M25_CHECK(cudaFuncGetAttributes(&pfa, k_panel_smem<R, false>));
+    M25_CHECK(cudaFuncGetAttributes(&pfa, k_panel_smem<R>));
     const int smem_cap = smem_optin - (int)pfa.sharedSizeBytes;      // less the kernel's static shared memory
-    M25_CHECK(cudaFuncSetAttribute(k_panel_smem<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_cap));
-    // The cluster panel (the exchange in distributed shared memory) takes the panels whose rows fit a cluster's
-    // blocks: as many blocks as the largest cluster this kernel can have on the device (16 where non-portable
-    // sizes are allowed), a block's rows and its records in its shared memory. M25_PANEL_CLUSTER=0: never.
-    int cl_max = 0, cl_rows_cap = 0;
+    M25_CHECK(cudaFuncSetAttribute(k_panel_smem<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_cap));
+    // The cluster panel (panel.cu) takes the panels whose rows fit its threads' registers. M25_PANEL_CLUSTER=0: never;
+    // M25_PANEL_CLUSTER_MAX caps the cluster.
+    int cl_max = 0;
     {
-        const char *e = getenv("M25_PANEL_CLUSTER");
-        if (!e || atoi(e) != 0) {
-            cudaFuncAttributes cfa;
-            M25_CHECK(cudaFuncGetAttributes(&cfa, k_panel_smem<R, true>));
-            const int cl_smem = smem_optin - (int)cfa.sharedSizeBytes;
-            M25_CHECK(cudaFuncSetAttribute(k_panel_smem<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cl_smem));
-            M25_CHECK(cudaFuncSetAttribute(k_panel_smem<R, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            cl_rows_cap = (int)(((size_t)cl_smem - sizeof(PanelRecords) - 16) / (sizeof(cpx<R>) * NB));
-            cudaLaunchConfig_t qc = {};
-            cudaLaunchAttribute qa[1];
-            qa[0].id = cudaLaunchAttributeClusterDimension;
-            qa[0].val.clusterDim.x = 16; qa[0].val.clusterDim.y = 1; qa[0].val.clusterDim.z = 1;
-            qc.gridDim = dim3(16); qc.blockDim = dim3(PANEL_THREADS); qc.dynamicSmemBytes = (size_t)cl_smem;
-            qc.attrs = qa; qc.numAttrs = 1;
-            int mc = 0;
-            if (cudaOccupancyMaxPotentialClusterSize(&mc, (void *)k_panel_smem<R, true>, &qc) != cudaSuccess) {
-                (void)cudaGetLastError();
-                mc = 0;
-            }
-            cl_max = std::min(16, mc);
-            if (const char *m = getenv("M25_PANEL_CLUSTER_MAX")) cl_max = std::min(cl_max, atoi(m));
-            if (cl_max < 2) cl_max = 0;
-        }
+        const char *e = getenv("M25_PANEL_CLUSTER"), *m = getenv("M25_PANEL_CLUSTER_MAX");
+        if (!e || atoi(e) != 0) cl_max = m25_panel_cluster_max(sizeof(R) == 4);
+        if (m) cl_max = std::min(cl_max, atoi(m));
+        if (cl_max < 2) cl_max = 0;
     }
     // Blocks of the panel: few enough that the cooperative launch finds its SMs quickly while the other stream's
     // update holds the rest (the exchange costs about the same from 37 to 148 blocks), but at least as many as
@@ -1967,25 +1878,17 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
             const size_t psmem = sizeof(cpx<R>) * (size_t)cs * jb;
             void *args[] = {&A, &lda, &n, (void *)&k0, (void *)&jb, &ipiv, &pw, &err};
             const int rows = n - k0;
-            if (cl_max && rows <= cl_max * cl_rows_cap) {               // one cluster, at least 64 rows a block
-                const int Gc = std::min(cl_max, std::max(2, (rows + 63) / 64));
-                const int csc = (rows + Gc - 1) / Gc;
-                cudaLaunchConfig_t lc = {};
-                cudaLaunchAttribute la1[1];
-                la1[0].id = cudaLaunchAttributeClusterDimension;
-                la1[0].val.clusterDim.x = (unsigned)Gc; la1[0].val.clusterDim.y = 1; la1[0].val.clusterDim.z = 1;
-                lc.gridDim = dim3(Gc); lc.blockDim = dim3(PANEL_THREADS);
-                lc.dynamicSmemBytes = ((size_t)csc * jb * sizeof(cpx<R>) + 15) / 16 * 16 + sizeof(PanelRecords);
-                lc.stream = H; lc.attrs = la1; lc.numAttrs = 1;
-                M25_CHECK(cudaLaunchKernelExC(&lc, (const void *)k_panel_smem<R, true>, args));
+            if (cl_max && rows <= m25_panel_cluster_rows(sizeof(R) == 4, cl_max)) {      // one cluster (panel.cu)
+                if ((rc = m25_panel_cluster(A, lda, n, k0, jb, ipiv, sizeof(R) == 4, cl_max, err, H))) return rc;
             } else if (psmem <= (size_t)smem_cap) {                    // (flagged records: no barrier to reset)
-                M25_CHECK(cudaLaunchCooperativeKernel((void *)k_panel_smem<R, false>, dim3(Gp), dim3(PANEL_THREADS),
+                M25_CHECK(cudaLaunchCooperativeKernel((void *)k_panel_smem<R>, dim3(Gp), dim3(PANEL_THREADS),
                                                       args, psmem, H));
+                m25_note_launch();
             } else {
                 M25_CHECK(cudaMemsetAsync(bar, 0, (2 + 2 * (size_t)G) * sizeof(unsigned), H));
                 M25_CHECK(cudaLaunchCooperativeKernel((void *)k_panel<R>, dim3(Gp), dim3(PANEL_THREADS), args, 0, H));
+                m25_note_launch();
             }
-            m25_note_launch();
             if ((rc = trsm(k0, jb, k0 + jb, KE, true, H))) return rc;     // the rest of the outer panel
             // in FP32 on the CUDA cores, not 3xTF32: the columns of L pass through every update of their outer
             // panel, and the tensor-core error there (about 2^-22 a product against 2^-24) costs the factor its
