@@ -1,0 +1,82 @@
+"""What is prepared once per factor and per frequency, at the sizes where the split changes: the solves' row permutation
+(interchanges resolved 256 at a time) and diagonal-block inverses (64 rows, joined from 16), the spline's tridiagonal
+system (two, or up to ten, equations a thread)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip('torch')
+
+
+def _solve(LU, ipiv, B, single):
+    from mom25d_b200 import _lib
+    from mom25d_b200._lib import P, check, lib
+    n, k = B.shape
+    aux = torch.empty(int(lib().m25_getrs_aux_bytes(n, int(single))), dtype=torch.uint8, device='cuda')
+    check(lib().m25_getrs_prepare(P(LU), ctypes.c_long(n), n, P(ipiv), int(single), P(aux), ctypes.c_size_t(aux.numel()),
+                                  _lib.stream_ptr()), 'prepare')
+    X = B.clone()
+    check(lib().m25_getrs_aux(P(LU), ctypes.c_long(n), n, int(single), P(aux), P(X), k, _lib.stream_ptr()), 'solve')
+    _lib.sync_check(what='solve')
+    return X
+
+
+@pytest.mark.parametrize('n', [1, 2, 15, 17, 63, 64, 65, 255, 256, 257, 511, 513, 1000])
+@pytest.mark.parametrize('kind', ['down', 'any', 'none'])
+def test_row_permutation(n, kind):
+    """With L = U = I the solve is the permutation alone: the interchanges applied from the last to the first."""
+    rng = np.random.default_rng(n)
+    i = np.arange(n)
+    piv = {'down': i + rng.integers(0, n - i), 'any': rng.integers(0, n, n), 'none': i}[kind].astype(np.int32)
+    B = rng.standard_normal((n, 2)) + 1j * rng.standard_normal((n, 2))
+    want = B.copy()
+    for r in range(n - 1, -1, -1):
+        want[[r, piv[r]]] = want[[piv[r], r]]
+    LU = torch.eye(n, dtype=torch.complex128, device='cuda')
+    X = _solve(LU, torch.from_numpy(piv).to('cuda'), torch.from_numpy(B).to('cuda'), False)
+    assert np.array_equal(X.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize('n', [1, 15, 16, 17, 33, 63, 64, 65, 130])
+@pytest.mark.parametrize('single', [True, False])
+def test_block_inverses(n, single):
+    """Solves by the diagonal-block inverses of a factor with full off-diagonal triangles, against the product."""
+    rng = np.random.default_rng(n)
+    F = (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / max(4.0, n ** 0.5)
+    F[np.arange(n), np.arange(n)] += 2.0
+    dt = torch.complex64 if single else torch.complex128
+    LU = torch.from_numpy(F.T.copy()).to('cuda').to(dt)                    # column-major F
+    Fq = LU.T.to(torch.complex128).cpu().numpy()
+    L, U = np.tril(Fq, -1) + np.eye(n), np.triu(Fq)
+    X0 = rng.standard_normal((n, 3)) + 1j * rng.standard_normal((n, 3))
+    Zt = (L @ U).T                                                         # Z X = B with A = Z^T = L U
+    B = torch.from_numpy(Zt @ X0).to('cuda').to(dt)
+    X = _solve(LU, torch.arange(n, dtype=torch.int32, device='cuda'), B, single).to(torch.complex128).cpu().numpy()
+    eps = 2.0 ** -24 if single else 2.0 ** -53
+    # |X - X0| <= c n eps cond(L) cond(U) |X0| with c = 16: forming B, the two inverses, the two products
+    bound = 16 * n * eps * np.linalg.cond(L) * np.linalg.cond(U) * np.linalg.norm(X0)
+    assert np.linalg.norm(X - X0) <= bound
+
+
+@pytest.mark.parametrize('n', [4, 5, 6, 7, 200, 260, 514, 515, 1030, 2300])
+def test_spline(n):
+    from scipy.interpolate import CubicSpline
+    from mom25d_b200 import _lib
+    from mom25d_b200._lib import P, check, lib
+    rng = np.random.default_rng(n)
+    x = 0.07 * np.linspace(0, 1, n) ** 2 if n % 2 == 0 else np.cumsum(rng.uniform(0.2, 1.0, n))
+    x = x - x[0]
+    y = np.exp(-9j * x / x[-1]) / (1 + np.arange(3)[:, None] + x / x[-1])
+    nf = 1000
+    dx = np.linspace(0, x[-1], nf)[1]
+    out = torch.empty((3, nf), dtype=torch.complex128, device='cuda')
+    d_x, d_y = _lib.dev(x), _lib.dev(y)
+    check(lib().m25_spline_uniform(P(d_x), P(d_y), 3, n, ctypes.c_double(dx), nf, P(out), 0,
+                                   ctypes.c_long(nf), ctypes.c_long(0), 1, _lib.stream_ptr()), 'm25_spline_uniform')
+    _lib.sync_check()
+    want = np.array([CubicSpline(x, r)(np.linspace(0, x[-1], nf)) for r in y])
+    # both solve the system to rounding: differences of a few hundred ulp of the largest sample (steep end pieces)
+    assert np.abs(out.cpu().numpy() - want).max() <= 1e-12
