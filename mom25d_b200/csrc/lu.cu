@@ -666,24 +666,18 @@ __global__ void __launch_bounds__(256) k_trsm(R *A, long lda, int k0, int jb, lo
 // columns are staged through shared memory (a column's stride NB + 1: the lanes' reads of their own columns fall in
 // different banks) so that every global load and store is a warp's 256 contiguous bytes. The arithmetic and its
 // order are those of k_trsm (row i's multiple subtracted from the rows below, i ascending).
-// With SWAP, the panel's own interchanges (ipiv[k0 .. k0 + NB)) are applied to the columns as they are loaded: the
-// solved rows come from the plan's sources, and the rows below that move are written back directly (the separate
-// interchange launch folded into this one).
-template <typename R, int T64_WARPS, bool SWAP>
-__global__ void __launch_bounds__(32 * T64_WARPS) k_trsm64(R *A, long lda, int k0, long c0, long c1, const int *ipiv,
-                                                           int n, int *err)
+template <typename R, int T64_WARPS>
+__global__ void __launch_bounds__(32 * T64_WARPS) k_trsm64(R *A, long lda, int k0, long c0, long c1)
 {
     typedef cpx<R> C;
     typedef typename vec2_of<R>::type V;
     constexpr int XS = NB + 1;
     extern __shared__ __align__(16) unsigned char t64_raw[];
-    __shared__ SwapPlan P;
     C *L = reinterpret_cast<C *>(t64_raw);                   // L[i * NB + k] = L11(k, i)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     C *Xs = L + NB * NB + (size_t)w * 32 * XS;
     const V *A2 = reinterpret_cast<const V *>(A);
     static_assert(NB * NB % (8 * 32 * T64_WARPS) == 0, "L11 in whole batches");
-    if (SWAP) swap_plan(ipiv, k0, NB, n, P, err);
     for (int e0 = threadIdx.x; e0 < NB * NB; e0 += 8 * 32 * T64_WARPS) {     // 8 loads in flight a thread
         V v[8];
 #pragma unroll
@@ -695,15 +689,7 @@ __global__ void __launch_bounds__(32 * T64_WARPS) k_trsm64(R *A, long lda, int k
         for (int q = 0; q < 8; ++q) L[e0 + q * 32 * T64_WARPS] = mk<R>(v[q].x, v[q].y);
     }
     const long cbase = c0 + ((long)blockIdx.x * T64_WARPS + w) * 32;
-    if (SWAP) {                                             // 4 rows x 8 (4) columns of loads in flight a lane
-        constexpr int SC = sizeof(R) == 4 ? 8 : 4;
-        for (int c8 = 0; c8 < 32; c8 += SC) {
-            long cs[SC];
-#pragma unroll
-            for (int j = 0; j < SC; ++j) cs[j] = cbase + c8 + j < c1 ? cbase + c8 + j : -1;
-            apply_plan<R, 4, SC>(A, lda, cs, P, lane, Xs + c8 * XS, NB, XS, 1);
-        }
-    } else for (int c8 = 0; c8 < 32; c8 += 8) {             // 16 loads in flight a lane
+    for (int c8 = 0; c8 < 32; c8 += 8) {             // 16 loads in flight a lane
         V v[8][2];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
@@ -770,14 +756,17 @@ template <typename R> constexpr size_t t64_smem()
     return sizeof(cpx<R>) * (NB * NB + (size_t)t64_warps<R>() * 32 * (NB + 1));
 }
 
-// U12 of a whole outer panel in one launch: rows [K0, K0 + JB) (JB <= NB2) of the columns [c0, c1), after the outer
-// panel's interchanges (ipiv[K0 .. K0 + JB), applied as a plan; the rows below that move written back directly),
+// U12 of a panel of up to NB2 columns in one launch: rows [K0, K0 + JB) of the columns [c0, c1), after the panel's
+// interchanges (ipiv[K0 .. K0 + JB), applied as a plan; the rows below that move written back directly),
 // U12 = L11^-1 A12 with L11 = A[K0 .., K0 ..] unit lower. TO_COLS columns a CTA of 256 threads (a warp a column),
 // their JB rows in shared memory. By 64-row blocks: the diagonal block of L11 staged in shared memory, each warp
 // solves its column's 64 rows (two rows a lane in registers, the solved value passed by shuffle), then every thread
 // takes a row below the block and subtracts the block's multiples from it for all the CTA's columns (L read from
-// the factor, coalesced across the threads). Each entry takes its terms x -= L(k, i) x_i in ascending i, as a
-// forward substitution does; FP32 (FP64) on the CUDA cores throughout.
+// the factor, coalesced across the threads, a batch ahead of its use, as the next diagonal block is). Each entry takes
+// its terms x -= L(k, i) x_i in ascending i, as a forward substitution does; FP32 (FP64) on the CUDA cores throughout.
+// Latency-bound: few columns, a chain of JB rows. In the complex64 LU of n = 4,977, 15 us on average over its 58 panels
+// of 64 (192 columns or fewer; a thread a column, k_trsm64, took 30) and 19 outer panels of 256 (66 with every entry of
+// L read where it is used).
 #define TO_COLS 8
 #define TO_THREADS 256
 static_assert(TO_COLS * 32 == TO_THREADS, "a warp a column");
@@ -788,61 +777,104 @@ __global__ void __launch_bounds__(TO_THREADS) k_trsm_outer(R *A, long lda, int n
                                                            long c0, long c1, int *err)
 {
     typedef cpx<R> C;
+    constexpr int LQ = NB * NB / TO_THREADS;               // entries of a diagonal block a thread
+    constexpr int CH = sizeof(R) == 4 ? 16 : 8;            // terms of a row below in flight
     extern __shared__ __align__(16) unsigned char to_raw[];
     __shared__ SwapPlan P;
     C *X = reinterpret_cast<C *>(to_raw);                 // X[r * TO_COLS + j]: row K0 + r of the CTA's column j
     C *Lb = X + (size_t)NB2 * TO_COLS;                     // Lb[i * (NB + 1) + k] = L11(kb + k, kb + i)
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const long cw = c0 + (long)blockIdx.x * TO_COLS + w;    // this warp's column
+    C lq[LQ];                                              // the next diagonal block on its way to Lb
+    auto fetch = [&](int kb) {
+        const int jb = min(NB, JB - kb);
+#pragma unroll
+        for (int q = 0; q < LQ; ++q) {
+            const int e = t + TO_THREADS * q, i = e / NB, k = e % NB;
+            lq[q] = i < jb && k < jb ? ldc<R>(A, (size_t)(K0 + kb + i) * lda + K0 + kb + k) : mk<R>(0, 0);
+        }
+    };
+    auto store = [&]() {
+#pragma unroll
+        for (int q = 0; q < LQ; ++q) {
+            const int e = t + TO_THREADS * q;
+            Lb[e / NB * (NB + 1) + e % NB] = lq[q];
+        }
+    };
+    fetch(0);
     swap_plan(ipiv, K0, JB, n, P, err);
     {
         long cs[1] = {cw < c1 ? cw : -1};
-        apply_plan<R, 2 * PLAN_MAX / 32, 1>(A, lda, cs, P, lane, X + w, JB, 0, TO_COLS);
+        if (JB <= NB) apply_plan<R, 2 * NB / 32, 1>(A, lda, cs, P, lane, X + w, JB, 0, TO_COLS);
+        else apply_plan<R, 2 * PLAN_MAX / 32, 1>(A, lda, cs, P, lane, X + w, JB, 0, TO_COLS);
         if (cw >= c1)
             for (int r = lane; r < JB; r += 32) X[r * TO_COLS + w] = mk<R>(0, 0);
     }
+    store();
+    __syncthreads();
     for (int kb = 0; kb < JB; kb += NB) {
         const int jb = min(NB, JB - kb);
-        __syncthreads();                                   // (X complete; the previous block's Lb reads done)
-        for (int e = t; e < jb * jb; e += TO_THREADS) {
-            const int i = e / jb, k = e % jb;
-            Lb[i * (NB + 1) + k] = ldc<R>(A, (size_t)(K0 + kb + i) * lda + K0 + kb + k);
-        }
-        __syncthreads();
+        const bool more = kb + jb < JB;                    // (then jb == NB)
+        if (more) fetch(kb + jb);
         {                                                  // the diagonal block, warp w's column
             C x0 = lane < jb ? X[(kb + lane) * TO_COLS + w] : mk<R>(0, 0);
             C x1 = lane + 32 < jb ? X[(kb + lane + 32) * TO_COLS + w] : mk<R>(0, 0);
-            for (int i = 0; i < jb - 1; ++i) {
-                const C s = i < 32 ? x0 : x1;
+#pragma unroll 4
+            for (int i = 0; i < min(32, jb - 1); ++i) {
                 C xi;
-                xi.x = __shfl_sync(0xffffffffu, s.x, i & 31);
-                xi.y = __shfl_sync(0xffffffffu, s.y, i & 31);
-                if (lane > i && lane < jb) cfms<R>(x0, Lb[i * (NB + 1) + lane], xi);
-                if (lane + 32 > i && lane + 32 < jb) cfms<R>(x1, Lb[i * (NB + 1) + lane + 32], xi);
+                xi.x = __shfl_sync(0xffffffffu, x0.x, i);
+                xi.y = __shfl_sync(0xffffffffu, x0.y, i);
+                if (lane > i) cfms<R>(x0, Lb[i * (NB + 1) + lane], xi);
+                cfms<R>(x1, Lb[i * (NB + 1) + lane + 32], xi);
+            }
+#pragma unroll 4
+            for (int i = 32; i < jb - 1; ++i) {
+                C xi;
+                xi.x = __shfl_sync(0xffffffffu, x1.x, i - 32);
+                xi.y = __shfl_sync(0xffffffffu, x1.y, i - 32);
+                if (lane + 32 > i) cfms<R>(x1, Lb[i * (NB + 1) + lane + 32], xi);
             }
             if (lane < jb) X[(kb + lane) * TO_COLS + w] = x0;
             if (lane + 32 < jb) X[(kb + lane + 32) * TO_COLS + w] = x1;
         }
         __syncthreads();
-        for (int r = kb + jb + t; r < JB; r += TO_THREADS) {   // the rows below the block
-            C x[TO_COLS];
+        if (!more) break;
+        const int r = kb + NB + t;                          // the rows below the block (at most NB2 - NB: one a thread)
+        if (r < JB) {
+            C x[TO_COLS], lv[CH];
+            uint4 *xr = reinterpret_cast<uint4 *>(X + r * TO_COLS);
+            constexpr int XQ = TO_COLS * (int)sizeof(C) / 16;
 #pragma unroll
-            for (int j = 0; j < TO_COLS; ++j) x[j] = X[r * TO_COLS + j];
+            for (int q = 0; q < XQ; ++q) reinterpret_cast<uint4 *>(x)[q] = xr[q];
             const R *lr = A + 2 * ((size_t)(K0 + kb) * lda + K0 + r);
-#pragma unroll 8
-            for (int i = 0; i < jb; ++i) {
-                const C l = ldc<R>(lr, (size_t)i * lda);
 #pragma unroll
-                for (int j = 0; j < TO_COLS; ++j) cfms<R>(x[j], l, X[(kb + i) * TO_COLS + j]);
+            for (int q = 0; q < CH; ++q) lv[q] = ldc<R>(lr, (size_t)q * lda);
+            for (int i = 0; i < NB; i += CH) {
+                C ln[CH];
+#pragma unroll
+                for (int q = 0; q < CH; ++q) ln[q] = i + CH < NB ? ldc<R>(lr, (size_t)(i + CH + q) * lda) : mk<R>(0, 0);
+#pragma unroll
+                for (int q = 0; q < CH; ++q) {
+                    C xi[TO_COLS];
+                    const uint4 *xp = reinterpret_cast<const uint4 *>(X + (kb + i + q) * TO_COLS);
+#pragma unroll
+                    for (int h = 0; h < XQ; ++h) reinterpret_cast<uint4 *>(xi)[h] = xp[h];
+#pragma unroll
+                    for (int j = 0; j < TO_COLS; ++j) cfms<R>(x[j], lv[q], xi[j]);
+                }
+#pragma unroll
+                for (int q = 0; q < CH; ++q) lv[q] = ln[q];
             }
 #pragma unroll
-            for (int j = 0; j < TO_COLS; ++j) X[r * TO_COLS + j] = x[j];
+            for (int q = 0; q < XQ; ++q) xr[q] = reinterpret_cast<uint4 *>(x)[q];
         }
+        store();                                           // (the diagonal block's reads of Lb ended at the barrier)
+        __syncthreads();
     }
-    __syncthreads();
     if (cw < c1)
         for (int r = lane; r < JB; r += 32) stc<R>(A, (size_t)cw * lda + K0 + r, X[r * TO_COLS + w]);
 }
+static_assert(NB2 - NB <= TO_THREADS, "a thread a row below the first block");
 
 // C (M x N) -= A (M x K) B (K x N), all column-major complex inside the factor (lda). A 128 x 64 tile per block of
 // 256 threads, each 8 x 4 outputs; K staged BK at a time through two shared-memory buffers, the next slice loaded
@@ -1855,9 +1887,7 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
     M25_CHECK(cudaMemsetAsync(pw.ll_cand, 0, ll_bytes, H));         // flags 0: no column's (they are column + 1)
     const size_t trsm_smem = sizeof(cpx<R>) * (NB * NB + NB * 64);
     M25_CHECK(cudaFuncSetAttribute(k_trsm<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem));
-    M25_CHECK(cudaFuncSetAttribute(k_trsm64<R, t64_warps<R>(), false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)t64_smem<R>()));
-    M25_CHECK(cudaFuncSetAttribute(k_trsm64<R, t64_warps<R>(), true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    M25_CHECK(cudaFuncSetAttribute(k_trsm64<R, t64_warps<R>()>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)t64_smem<R>()));
     M25_CHECK(cudaFuncSetAttribute(k_trsm_outer<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)to_smem<R>()));
     int smem_optin = 0, dev = 0;
@@ -1897,28 +1927,22 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
         M25_LAUNCH_CHECK("k_laswp_plan");
         return M25_OK;
     };
-    // U12 rows k0 .. k0 + jb of the columns [c0, c1); swap: the panel's interchanges applied to them on the way
-    auto trsm = [&](int k0, int jb, long c0, long c1, bool swap, cudaStream_t cs) -> int {
+    // U12 rows k0 .. k0 + jb of the columns [c0, c1), their interchanges applied before
+    auto trsm = [&](int k0, int jb, long c0, long c1, cudaStream_t cs) -> int {
         if (c1 <= c0) return M25_OK;
         if (jb == NB) {
             const long per = 32L * t64_warps<R>();
-            const unsigned grid = (unsigned)((c1 - c0 + per - 1) / per);
-            if (swap)
-                k_trsm64<R, t64_warps<R>(), true><<<grid, (unsigned)per, t64_smem<R>(), cs>>>(A, lda, k0, c0, c1,
-                                                                                               ipiv, n, err);
-            else
-                k_trsm64<R, t64_warps<R>(), false><<<grid, (unsigned)per, t64_smem<R>(), cs>>>(A, lda, k0, c0, c1,
-                                                                                                ipiv, n, err);
+            k_trsm64<R, t64_warps<R>()><<<(unsigned)((c1 - c0 + per - 1) / per), (unsigned)per, t64_smem<R>(), cs>>>(
+                A, lda, k0, c0, c1);
             M25_LAUNCH_CHECK("k_trsm64");
             return M25_OK;
         }
-        int rc2;
-        if (swap && (rc2 = laswp(k0, jb, c0, c1, 0, 0, 0, 1, cs))) return rc2;
         k_trsm<R><<<(c1 - c0 + 63) / 64, 256, trsm_smem, cs>>>(A, lda, k0, jb, c0, c1);
         M25_LAUNCH_CHECK("k_trsm");
         return M25_OK;
     };
-    // U12 of the whole outer panel [K0, K0 + JB) on the columns [c0, c1), its interchanges applied on the way
+    // U12 of the panel [K0, K0 + JB) (a panel, or the whole outer panel) on the columns [c0, c1), its interchanges
+    // applied on the way: a warp a column, for the few columns of the critical path
     auto trsm_outer = [&](int K0, int JB, long c0, long c1, cudaStream_t cs) -> int {
         if (c1 <= c0) return M25_OK;
         k_trsm_outer<R><<<(unsigned)((c1 - c0 + TO_COLS - 1) / TO_COLS), TO_THREADS, to_smem<R>(), cs>>>(
@@ -1983,7 +2007,7 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
                 M25_CHECK(cudaLaunchCooperativeKernel((void *)k_panel<R>, dim3(Gp), dim3(PANEL_THREADS), args, 0, H));
                 m25_note_launch();
             }
-            if ((rc = trsm(k0, jb, k0 + jb, KE, true, H))) return rc;     // the rest of the outer panel
+            if ((rc = trsm_outer(k0, jb, k0 + jb, KE, H))) return rc;      // the rest of the outer panel
             // in FP32 on the CUDA cores, not 3xTF32: the columns of L pass through every update of their outer
             // panel, and the tensor-core error there (about 2^-22 a product against 2^-24) costs the factor its
             // use as a preconditioner near the low-frequency end (fresh LUs at 0.67 and 0.91 GHz of the routed
@@ -2005,7 +2029,7 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
         if (KE2 < n) {
             for (int k0 = K0; k0 < KE; k0 += NB) {
                 const int jb = std::min(NB, KE - k0);
-                if ((rc = trsm(k0, jb, KE2, n, false, Lo))) return rc;
+                if ((rc = trsm(k0, jb, KE2, n, Lo))) return rc;
                 if ((rc = gemm(k0 + jb, KE - k0 - jb, KE2, n - KE2, k0, jb, true, Lo))) return rc;
             }
             if ((rc = gemm(KE, n - KE, KE2, KE3 - KE2, K0, JB, true, Lo))) return rc;   // block k + 2's columns
