@@ -20,50 +20,76 @@ __device__ __forceinline__ void tab_rest(const TB &tb, int t, R r, cpx<R> &ga, c
     gq = q0 * (1 - f) + q1 * f;
 }
 
+// 1 / sqrt(x); double: CUDA's rsqrt (1 ulp), a third of a root and a division
+__device__ __forceinline__ double inv_root(double x) { return rsqrt(x); }
+__device__ __forceinline__ float inv_root(float x) { return 1.0f / sqrtf(x); }
+
+// The kernel at the squared distance d2: one reciprocal root gives 1 / r and r (with a Newton step: r to rounding), one
+// more the image's or the other interface's 1 / R (four divisions by r, a division and a root of their own before)
 template <typename R, typename TB>
-__device__ __forceinline__ void tab_kern(const TB &tb, int la, int lb, R r, cpx<R> &ga, cpx<R> &gq)
+__device__ __forceinline__ void tab_kern(const TB &tb, int la, int lb, R d2, cpx<R> &ga, cpx<R> &gq)
 {
-    int t = tb.tab[la * tb.L + lb];
+    const int t = tb.tab[la * tb.L + lb];
+    const R ir = d2 > 0 ? inv_root(d2) : (R)0;
+    R r = d2 * ir;
+    r = fma(fma(-r, r, d2), (R)0.5 * ir, r);
     tab_rest<R>(tb, t, r, ga, gq);
-    int kd = tb.kind[t];
+    const int kd = tb.kind[t];
     if (kd == 0) {
-        if (r > 0) {
-            ga += ldc<R>((const R *)tb.cA, t) / r;
-            gq += ldc<R>((const R *)tb.cq, t) / r;
-        }
-        R di = (R)tb.dimg[t];
+        const cpx<R> ca = ldc<R>((const R *)tb.cA, t), cq = ldc<R>((const R *)tb.cq, t);
+        ga.x = fma(ca.x, ir, ga.x); ga.y = fma(ca.y, ir, ga.y);
+        gq.x = fma(cq.x, ir, gq.x); gq.y = fma(cq.y, ir, gq.y);
+        const R di = (R)tb.dimg[t];
         if (di > 0) {
-            R ri = (R)1 / sqrt(r * r + di * di);
-            ga += ldc<R>((const R *)tb.cAi, t) * ri;
-            gq += ldc<R>((const R *)tb.cqi, t) * ri;
+            const R ri = inv_root(fma(di, di, d2));
+            const cpx<R> ci = ldc<R>((const R *)tb.cAi, t), cj = ldc<R>((const R *)tb.cqi, t);
+            ga.x = fma(ci.x, ri, ga.x); ga.y = fma(ci.y, ri, ga.y);
+            gq.x = fma(cj.x, ri, gq.x); gq.y = fma(cj.y, ri, gq.y);
         }
     } else if (kd == 1) {
-        R dd = (R)tb.d[t];
-        R ri = (R)1 / sqrt(r * r + dd * dd);
-        ga += ldc<R>((const R *)tb.cA, t) * ri;
-        gq += ldc<R>((const R *)tb.cq, t) * ri;
+        const R dd = (R)tb.d[t], ri = inv_root(fma(dd, dd, d2));
+        const cpx<R> ca = ldc<R>((const R *)tb.cA, t), cq = ldc<R>((const R *)tb.cq, t);
+        ga.x = fma(ca.x, ri, ga.x); ga.y = fma(ca.y, ri, ga.y);
+        gq.x = fma(cq.x, ri, gq.x); gq.y = fma(cq.y, ri, gq.y);
     }
 }
 
-// centroid distance: the differences in double (nearby triangles' coordinates cancel), the root in R
+// squared centroid distance: the differences in double (nearby triangles' coordinates cancel)
 template <typename R>
-__device__ __forceinline__ R cdist(const double *c, int p, int q)
+__device__ __forceinline__ R cdist2(const double *c, int p, int q)
 {
-    double dx = c[2 * p] - c[2 * q], dy = c[2 * p + 1] - c[2 * q + 1];
-    return sqrt((R)(dx * dx + dy * dy));
+    const double dx = c[2 * p] - c[2 * q], dy = c[2 * p + 1] - c[2 * q + 1];
+    return (R)(dx * dx + dy * dy);
 }
 
 // ---- far field: fill_far (mom25d_core.cpp:132-173) ----------------------------------------------------------------
 // A 32 x 32 tile of edges per block. The reference evaluates the tabulated kernel 4 times per entry (one per pair
 // of the two edges' triangles); here the tile's distinct row and column triangles are found first (about 31 of
-// each for 32 edges), the kernel is evaluated once per distinct triangle pair into shared memory, and every entry
-// is assembled from four shared-memory lookups (0.95 evaluations an entry instead of 4). Each entry (m, n) is
-// formed in the reference's order for the pair (min(m, n), max(m, n)) and the kernel is symmetric in its two
-// triangles (distance, symmetric table map), so Z is exactly symmetric, as the reference writes it. A tile whose
-// distinct pairs do not fit the shared-memory budget evaluates its entries directly.
-struct EdgeHalves { int p[2]; int lt[2]; double a[2], dx[2], dy[2]; };
+// each for 32 edges), the kernel is evaluated once per distinct triangle pair into shared memory (a warp a row
+// triangle, a lane a column triangle), and every entry is assembled from shared-memory lookups:
+//   Z = jw sum_st (a_s d_s . a_t d_t) G_A + 4 / jw sum_st a_s a_t G_q,
+// the sums with real weights. The kernel is symmetric in its two triangles (distance, symmetric table map), so Z is
+// symmetric and only the tiles on and above the diagonal are computed; each is written twice, the second time
+// transposed through shared memory (0.5 evaluations an entry). On the diagonal tiles an entry below the diagonal is
+// formed as its mirror image is, so Z is exactly symmetric there too. A tile whose distinct pairs do not fit the
+// shared-memory budget evaluates its entries directly.
+// Bound by FP64 instructions and the tables' gathers (about 96 bytes of L2 sectors an evaluation). Ne = 8,508: 2.22 ms
+// with every tile computed, divisions by r and 4 complex products an entry, 1.44 ms so; Ne = 18,763: 11.0 -> 6.9 ms
+// (5.6 GB written: 0.85 ms).
+struct EdgeHalves { int p[2]; int lt[2]; double a[2], ax[2], ay[2]; };    // a = +-l / 2A x A; a times (centroid - vertex)
 
 #define FF_SMEM (48 * 1024)
+
+// tile `idx` of the tiles on and above the diagonal of an nt x nt grid, by rows
+__device__ __forceinline__ void upper_tile(long idx, int nt, int &by, int &bx)
+{
+    const double h = nt + 0.5;
+    by = (int)(h - sqrt(fmax(0.0, h * h - 2.0 * (double)idx)));
+    auto first = [&](int y) { return (long)y * nt - (long)y * (y - 1) / 2; };   // tiles before row y
+    while (by > 0 && first(by) > idx) --by;
+    while (by + 1 < nt && first(by + 1) <= idx) ++by;
+    bx = by + (int)(idx - first(by));
+}
 
 template <typename R, typename TB>
 __device__ __forceinline__ void fill_far_tile(R *Z, long ld, const m25_mesh &g, const TB &tb, double w)
@@ -72,13 +98,16 @@ __device__ __forceinline__ void fill_far_tile(R *Z, long ld, const m25_mesh &g, 
     extern __shared__ __align__(16) unsigned char ff_raw[];
     constexpr int GCAP = FF_SMEM / (2 * sizeof(C));                   // distinct triangle pairs a tile holds
     C *gas = reinterpret_cast<C *>(ff_raw), *gqs = gas + GCAP;
+    static_assert(32 * 33 * sizeof(C) <= FF_SMEM, "the transposed tile in the pairs' memory");
     __shared__ EdgeHalves rows[32], cols[32];
     __shared__ short uid[2][64];                                      // [row / col][edge half 2 e + s] -> distinct index
     __shared__ int tri[2][64];                                        // distinct triangles, in first-seen order
     __shared__ unsigned rep_mask[2][2];
     __shared__ int nu[2];
-    const int M0 = blockIdx.y * 32, N0 = blockIdx.x * 32;
-    const int tid = threadIdx.y * 32 + threadIdx.x;
+    int by, bx;
+    upper_tile(blockIdx.x, (g.Ne + 31) / 32, by, bx);
+    const int M0 = by * 32, N0 = bx * 32;
+    const int lane = threadIdx.x, wid = threadIdx.y, tid = wid * 32 + lane;
     if (tid < 64) {
         int e = (tid < 32 ? M0 : N0) + (tid & 31);
         EdgeHalves h;
@@ -87,10 +116,10 @@ __device__ __forceinline__ void fill_far_tile(R *Z, long ld, const m25_mesh &g, 
             h.p[0] = pp; h.p[1] = pm;
             h.lt[0] = g.lt[pp]; h.lt[1] = g.lt[pm];
             h.a[0] = g.ap[e] * g.area[pp]; h.a[1] = g.am[e] * g.area[pm];
-            h.dx[0] = g.cent[2 * pp] - g.vp[2 * e]; h.dy[0] = g.cent[2 * pp + 1] - g.vp[2 * e + 1];
-            h.dx[1] = g.cent[2 * pm] - g.vm[2 * e]; h.dy[1] = g.cent[2 * pm + 1] - g.vm[2 * e + 1];
+            h.ax[0] = h.a[0] * (g.cent[2 * pp] - g.vp[2 * e]); h.ay[0] = h.a[0] * (g.cent[2 * pp + 1] - g.vp[2 * e + 1]);
+            h.ax[1] = h.a[1] * (g.cent[2 * pm] - g.vm[2 * e]); h.ay[1] = h.a[1] * (g.cent[2 * pm + 1] - g.vm[2 * e + 1]);
         } else {
-            h.p[0] = h.p[1] = 0; h.lt[0] = h.lt[1] = 0; h.a[0] = h.a[1] = 0; h.dx[0] = h.dx[1] = h.dy[0] = h.dy[1] = 0;
+            h.p[0] = h.p[1] = 0; h.lt[0] = h.lt[1] = 0; h.a[0] = h.a[1] = 0; h.ax[0] = h.ax[1] = h.ay[0] = h.ay[1] = 0;
         }
         (tid < 32 ? rows : cols)[tid & 31] = h;
     }
@@ -120,61 +149,76 @@ __device__ __forceinline__ void fill_far_tile(R *Z, long ld, const m25_mesh &g, 
     const int nr = nu[0], nc = nu[1];
     const bool tabled = nr * nc <= GCAP;
     if (tabled) {
-        for (int q = tid; q < nr * nc; q += 256) {
-            const int i = q / nc, j = q - i * nc, p = tri[0][i], t = tri[1][j];
-            C ga, gq;
-            tab_kern<R>(tb, g.lt[p], g.lt[t], cdist<R>(g.cent, p, t), ga, gq);
-            gas[q] = ga;
-            gqs[q] = gq;
+        for (int j = lane; j < nc; j += 32) {
+            const int t = tri[1][j], lb = g.lt[t];
+            for (int i = wid; i < nr; i += 8) {
+                const int p = tri[0][i];
+                C ga, gq;
+                tab_kern<R>(tb, g.lt[p], lb, cdist2<R>(g.cent, p, t), ga, gq);
+                gas[i * nc + j] = ga;
+                gqs[i * nc + j] = gq;
+            }
         }
     }
     __syncthreads();
-    const int n = N0 + threadIdx.x;
-    if (n >= g.Ne) return;
-    const C jw = mk<R>(0, (R)w);
-    const C inv_jw = mk<R>(0, (R)(-1.0 / w));
-    for (int i = threadIdx.y; i < 32; i += 8) {
-        const int m = M0 + i;
-        if (m >= g.Ne) break;
-        const bool up = m <= n;
-        const EdgeHalves &A = up ? rows[i] : cols[threadIdx.x];
-        const EdgeHalves &B = up ? cols[threadIdx.x] : rows[i];
-        C v = mk<R>(0, 0);
-        for (int s = 0; s < 2; ++s)
-            for (int t = 0; t < 2; ++t) {
+    const int n = N0 + lane;
+    const R wr = (R)w, qw = (R)(4.0 / w);
+    const EdgeHalves &B = cols[lane];
+    C val[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = wid + 8 * k, m = M0 + i;
+        const EdgeHalves &A = rows[i];
+        const bool up = m <= n;                           // else the terms in the mirror image's order
+        C sa = mk<R>(0, 0), sq = mk<R>(0, 0);
+#pragma unroll
+        for (int s2 = 0; s2 < 2; ++s2)
+#pragma unroll
+            for (int t2 = 0; t2 < 2; ++t2) {
+                const int s = up ? s2 : t2, t = up ? t2 : s2;          // the row edge's half, the column edge's
                 C ga, gq;
                 if (tabled) {
-                    // the row-side index of the pair is the row edge's half, whichever of A, B that is
-                    const int ir = up ? uid[0][2 * i + s] : uid[0][2 * i + t];
-                    const int ic = up ? uid[1][2 * threadIdx.x + t] : uid[1][2 * threadIdx.x + s];
-                    ga = gas[ir * nc + ic];
-                    gq = gqs[ir * nc + ic];
+                    const int q = uid[0][2 * i + s] * nc + uid[1][2 * lane + t];
+                    ga = gas[q];
+                    gq = gqs[q];
                 } else {
-                    tab_kern<R>(tb, A.lt[s], B.lt[t], cdist<R>(g.cent, A.p[s], B.p[t]), ga, gq);
+                    tab_kern<R>(tb, A.lt[s], B.lt[t], cdist2<R>(g.cent, A.p[s], B.p[t]), ga, gq);
                 }
-                R dot = (R)A.dx[s] * (R)B.dx[t] + (R)A.dy[s] * (R)B.dy[t];
-                C term = (jw * dot) * ga + (gq * (R)4) * inv_jw;
-                v += ((R)A.a[s] * (R)B.a[t]) * term;
+                const R c = (R)A.ax[s] * (R)B.ax[t] + (R)A.ay[s] * (R)B.ay[t], q = (R)A.a[s] * (R)B.a[t];
+                sa.x = fma(c, ga.x, sa.x); sa.y = fma(c, ga.y, sa.y);
+                sq.x = fma(q, gq.x, sq.x); sq.y = fma(q, gq.y, sq.y);
             }
-        stc<R>(Z, (size_t)m * ld + n, v);
+        val[k] = mk<R>(qw * sq.y - wr * sa.y, wr * sa.x - qw * sq.x);
+        if (m < g.Ne && n < g.Ne) stc<R>(Z, (size_t)m * ld + n, val[k]);
+    }
+    if (by == bx) return;                                 // (the whole block)
+    __syncthreads();                                      // the pairs' memory becomes the tile's
+    C *tile = gas;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) tile[(wid + 8 * k) * 33 + lane] = val[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = wid + 8 * k;                        // row N0 + i of Z, column M0 + lane
+        if (N0 + i < g.Ne && M0 + lane < g.Ne) stc<R>(Z, (size_t)(N0 + i) * ld + M0 + lane, tile[lane * 33 + i]);
     }
 }
 
 // four CTAs an SM (64 registers; 88 let two): the tile's phases end in barriers, and the other CTAs' warps fill
-// those stalls (routed board, N = 18,788: the FP64 fill phase 15.5 -> 12.3 ms; three CTAs 12.6)
+// those stalls
 template <typename R, typename TB>
 __global__ void __launch_bounds__(256, 4) k_fill_far(R *Z, long ld, m25_mesh g, TB tb, double w)
 {
     fill_far_tile<R, TB>(Z, ld, g, tb, w);
 }
 
-// Several frequencies of one board in one launch: grid z is the frequency, each with its own Z, tables and w (the
+// Several frequencies of one board in one launch: grid y is the frequency, each with its own Z, tables and w (the
 // batched sweep: the far part of every frequency's Z, the tables of all of them resident).
 template <typename R, typename TB>
 __global__ void __launch_bounds__(256, 4) k_fill_far_multi(R *const *Zs, long ld, m25_mesh g, const TB *tbs,
                                                         const double *ws)
 {
-    const int f = blockIdx.z;
+    const int f = blockIdx.y;
     const TB tb = tbs[f];
     fill_far_tile<R, TB>(Zs[f], ld, g, tb, ws[f]);
 }
@@ -199,7 +243,7 @@ __global__ void k_far_block(const int *R_, int nr, const int *C_, int nc, double
     for (int s = 0; s < 2; ++s)
         for (int t = 0; t < 2; ++t) {
             zd ga, gq;
-            tab_kern<double>(tb, g.lt[pm[s]], g.lt[pn[t]], cdist<double>(g.cent, pm[s], pn[t]), ga, gq);
+            tab_kern<double>(tb, g.lt[pm[s]], g.lt[pn[t]], cdist2<double>(g.cent, pm[s], pn[t]), ga, gq);
             zd term = (jw * (dx[s] * ex[t] + dy[s] * ey[t])) * ga + (gq * 4.0) * inv_jw;
             v += (am_[s] * an[t]) * term;
         }
@@ -355,7 +399,7 @@ __global__ void __launch_bounds__(256) k_near(int mode, Zt *Z, long ld, int *ri,
     // minus the centroid-rule value of the far fill
     {
         zd ga, gq;
-        tab_kern<double>(tb, la, lb, cdist<double>(g.cent, p, qq), ga, gq);
+        tab_kern<double>(tb, la, lb, cdist2<double>(g.cent, p, qq), ga, gq);
         const double wt = g.area[p] * g.area[qq];
         const double ox = g.cent[2 * p], oy = g.cent[2 * p + 1], sx = g.cent[2 * qq], sy = g.cent[2 * qq + 1];
         ga = ga * wt;
@@ -450,7 +494,7 @@ __global__ void k_fan_q(const int *F, int nf, double *out, m25_mesh g, m25_table
     if (idx >= (long)g.Nt * nf) return;
     int t = idx / nf, j = idx % nf, f = F[j];
     zd ga, gq;
-    tab_kern<double>(tb, g.lt[t], g.lt[f], cdist<double>(g.cent, t, f), ga, gq);
+    tab_kern<double>(tb, g.lt[t], g.lt[f], cdist2<double>(g.cent, t, f), ga, gq);
     stc<double>(out, idx, gq * (g.area[t] * g.area[f]));
 }
 
@@ -511,6 +555,7 @@ __global__ void __launch_bounds__(128) k_mv_pairs(int K, m25_mesh g, m25_tables 
     const double cx = live ? g.cent[2 * p] : 0, cy = live ? g.cent[2 * p + 1] : 0;
     const int lp = live ? g.lt[p] : 0;
     zd ax[KMAX], ay[KMAX], aq[KMAX];
+#pragma unroll
     for (int c = 0; c < KMAX; ++c) ax[c] = ay[c] = aq[c] = mk<double>(0, 0);
     // this block's chunk of source triangles (grid.y chunks; partial sums added atomically)
     const int chunk = (g.Nt + gridDim.y - 1) / gridDim.y;
@@ -535,7 +580,7 @@ __global__ void __launch_bounds__(128) k_mv_pairs(int K, m25_mesh g, m25_tables 
         for (int j = 0; j < qn; ++j) {
             double dx = cx - sc[j][0], dy = cy - sc[j][1];
             zd ga, gq;
-            tab_kern<double>(tb, lp, sl[j], sqrt(dx * dx + dy * dy), ga, gq);
+            tab_kern<double>(tb, lp, sl[j], dx * dx + dy * dy, ga, gq);
 #pragma unroll
             for (int c = 0; c < KMAX; ++c) {
                 if (c < K) { ax[c] += ga * SX[j][c]; ay[c] += ga * SY[j][c]; aq[c] += gq * S0[j][c]; }
@@ -543,7 +588,9 @@ __global__ void __launch_bounds__(128) k_mv_pairs(int K, m25_mesh g, m25_tables 
         }
     }
     if (!live) return;
-    for (int c = 0; c < K; ++c) {
+#pragma unroll
+    for (int c = 0; c < KMAX; ++c) {                       // (a constant trip count: the sums stay in registers)
+        if (c >= K) break;
         size_t o = 2 * ((size_t)p * K + c);
         atomicAdd(vAx + o, ax[c].x); atomicAdd(vAx + o + 1, ax[c].y);
         atomicAdd(vAy + o, ay[c].x); atomicAdd(vAy + o + 1, ay[c].y);
@@ -621,7 +668,8 @@ extern "C" int m25_fill_far(void *d_Z, long ld, int single, const m25_mesh *g, c
 {
     M25_REQUIRE(d_Z && g && ld >= g->Ne, "m25_fill_far: Z, g and ld >= Ne required");
     if (g->Ne == 0) return M25_OK;
-    dim3 grid((g->Ne + 31) / 32, (g->Ne + 31) / 32), block(32, 8);
+    const long nt = (g->Ne + 31) / 32;
+    const dim3 grid((unsigned)(nt * (nt + 1) / 2)), block(32, 8);      // the tiles on and above the diagonal
     if (single) {
         M25_REQUIRE(tbf, "m25_fill_far: single precision needs the complex64 tables");
         M25_CHECK(cudaFuncSetAttribute(k_fill_far<float, m25_tables_f>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -643,7 +691,8 @@ extern "C" int m25_fill_far_multi(void *const *d_Zs, long ld, int single, const 
     M25_REQUIRE(d_Zs && g && d_tables && d_w && ld >= g->Ne && nf >= 1 && nf <= 65535,
                 "m25_fill_far_multi: Zs, g, tables, w, ld >= Ne, 1 <= nf <= 65535");
     if (g->Ne == 0) return M25_OK;
-    dim3 grid((g->Ne + 31) / 32, (g->Ne + 31) / 32, nf), block(32, 8);
+    const long nt = (g->Ne + 31) / 32;
+    const dim3 grid((unsigned)(nt * (nt + 1) / 2), nf), block(32, 8);
     if (single) {
         M25_CHECK(cudaFuncSetAttribute(k_fill_far_multi<float, m25_tables_f>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, FF_SMEM));
