@@ -959,6 +959,83 @@ __global__ void __launch_bounds__(256) k_gemm_update(R *Cm, const R *Am, const R
     }
 }
 
+// The same for K <= 64 in complex64 (the updates inside an outer panel, at most 192 columns wide): the whole depth of
+// both operands is copied into shared memory at once (cp.async, 8 bytes: a factor's columns need not be 16-byte aligned)
+// in four groups of 16, the products of a group start as it lands, and C is read ahead of them. BM rows x 64 columns a
+// block of 256 threads, each BM / 16 x 4 outputs; BM = 64 where 128 rows a block would leave SMs idle. Each entry takes
+// its terms in k order, as k_gemm_update adds them. What bounds it is one SM's FP32 rate (8 us for 128 x 64 x 64).
+// n = 4,977: 24 us an update by k_gemm_update (slices of 8, rows of C 16 bytes at a time), 13 with BM = 64 (M below
+// about 4,700 rows), 19 with BM = 128 (above).
+__device__ __forceinline__ void cp_async8_zfill(void *smem, const void *gmem, bool valid)
+{
+    unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(sa), "l"(gmem), "r"(valid ? 8 : 0) : "memory");
+}
+constexpr size_t g64_smem(int bm) { return sizeof(cpx<float>) * 64 * ((size_t)bm + 65); }
+
+template <int BM>
+__global__ void __launch_bounds__(256) k_gemm64(float *Cm, const float *Am, const float *Bm, long lda, int M, int N, int K)
+{
+    typedef cpx<float> C;
+    constexpr int BN = 64, KG = 16, TI = BM / 16;
+    extern __shared__ __align__(16) unsigned char g64_raw[];
+    C(*As)[BM] = reinterpret_cast<C(*)[BM]>(g64_raw);                                // [64][BM]
+    C(*Bs)[BN + 1] = reinterpret_cast<C(*)[BN + 1]>(g64_raw + sizeof(C) * 64 * BM);  // [64][BN + 1]
+    const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const C *A2 = reinterpret_cast<const C *>(Am), *B2 = reinterpret_cast<const C *>(Bm);
+#pragma unroll
+    for (int g = 0; g < 64; g += KG) {
+        for (int e = t; e < KG * BM; e += 256) {
+            const int k = g + e / BM, m = e % BM;
+            const bool ok = k < K && m0 + m < M;
+            cp_async8_zfill(&As[k][m], A2 + (ok ? (size_t)k * lda + m0 + m : 0), ok);
+        }
+        for (int e = t; e < KG * BN; e += 256) {
+            const int k = g + e % KG, nn = e / KG;
+            const bool ok = k < K && n0 + nn < N;
+            cp_async8_zfill(&Bs[k][nn], B2 + (ok ? (size_t)(n0 + nn) * lda + k : 0), ok);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    C cv[TI][4], acc[TI][4];
+#pragma unroll
+    for (int i = 0; i < TI; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int m = m0 + tx + 16 * i, nn = n0 + ty + 16 * j;
+            cv[i][j] = m < M && nn < N ? ldc<float>(Cm, (size_t)nn * lda + m) : mk<float>(0, 0);
+            acc[i][j] = mk<float>(0, 0);
+        }
+#pragma unroll
+    for (int g = 0; g < 64; g += KG) {
+        if (g == 0) asm volatile("cp.async.wait_group 3;" ::: "memory");
+        else if (g == KG) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else if (g == 2 * KG) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+#pragma unroll 4
+        for (int k = g; k < g + KG; ++k) {
+            C a[TI], b[4];
+#pragma unroll
+            for (int i = 0; i < TI; ++i) a[i] = As[k][tx + 16 * i];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = Bs[k][ty + 16 * j];
+#pragma unroll
+            for (int i = 0; i < TI; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) cfma<float>(acc[i][j], a[i], b[j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < TI; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int m = m0 + tx + 16 * i, nn = n0 + ty + 16 * j;
+            if (m < M && nn < N) stc<float>(Cm, (size_t)nn * lda + m, cv[i][j] - acc[i][j]);
+        }
+}
+
 // The complex128 update C -= A B on the FP64 tensor cores (mma.sync m8n8k4 f64; Blackwell's tcgen05 has no FP64
 // kind). Column-major A (M x K), B (K x N), C (M x N), one leading dimension. A 64 x 64 tile a CTA of four warps,
 // each warp 32 x 32 complex: 2 x 4 tiles of 16 x 8 (mma m16n8k8) for the real and the imaginary part,
@@ -1914,6 +1991,8 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
     const int rows_cap = (int)((size_t)smem_cap / (sizeof(cpx<R>) * NB));   // a block's rows in shared memory
     const int gcap = std::min(G, PANEL_THREADS);                     // a thread of each block reads a block's record
     M25_CHECK(cudaFuncSetAttribute(k_gemm_update<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<R>()));
+    M25_CHECK(cudaFuncSetAttribute(k_gemm64<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g64_smem(64)));
+    M25_CHECK(cudaFuncSetAttribute(k_gemm64<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g64_smem(128)));
     M25_CHECK(cudaFuncSetAttribute(k_zgemm_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zdmma_smem()));
     // the interchanges ipiv[r0 .. r0 + nsw) on the columns [a0, a1) and [b0, b1); groups > 1: group g takes the
     // rows, count and first range shifted by g gs
@@ -1968,6 +2047,16 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
             return M25_OK;
         }
         dim3 grid((Nc + 63) / 64, (M + 127) / 128);
+        if constexpr (sizeof(R) == 4) {
+            if (K <= 64) {
+                if (2 * grid.x * grid.y <= (unsigned)G)
+                    k_gemm64<64><<<dim3(grid.x, (M + 63) / 64), 256, g64_smem(64), cs>>>(C22, L21, U12, lda, M, Nc, K);
+                else
+                    k_gemm64<128><<<grid, 256, g64_smem(128), cs>>>(C22, L21, U12, lda, M, Nc, K);
+                M25_LAUNCH_CHECK("k_gemm64");
+                return M25_OK;
+            }
+        }
         k_gemm_update<R><<<grid, 256, gemm_smem<R>(), cs>>>(C22, L21, U12, lda, M, Nc, K);
         M25_LAUNCH_CHECK("k_gemm_update");
         return M25_OK;
