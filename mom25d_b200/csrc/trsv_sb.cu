@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -43,13 +44,13 @@
 #define SB_KTS (SB / SB_KT)    // tiles a task
 #define SB_TS 72               // tile row stride (complex): 576 bytes; complex64 rows 16 words apart on the banks
 #define SB_NT 512              // threads of the solve kernel
-#define SB_TPR (SB_NT / SBC)   // threads a chunk row (16)
+#define SB_RPW 2               // chunk rows a warp
 #define SB_CHMAX 12            // chunks a CTA at most
 #define SB_NR 8                // right-hand sides a solve
 #define SB_MIN_N 2048          // smallest n solved this way (below it the chain of 64-row blocks is short)
 #define SB_GA 24               // CTAs on the chain's products: 8 chunks x 3 blocks in flight (y, u, w)
 static_assert(SBC * SB_NR <= SB_NT, "a chunk's entries one a thread");
-static_assert(SB_TPR == 16 && SB_KT % SB_TPR == 0, "16 threads a chunk row, whole terms a tile");
+static_assert(SB_RPW * (SB_NT / 32) == SBC && SB_KT % 32 == 0, "a chunk's rows over the warps, whole terms a tile");
 
 template <typename R> constexpr int sb_xs() { return 36 * 4 / (int)sizeof(cpx<R>); }    // staged vector row stride
 // shared memory of the solve kernel with a ring of nbuf tiles
@@ -249,75 +250,80 @@ struct SbSolve {
     const int *epoch_ptr; int *err;
 };
 
-// acc[c] += sum_{kk < 64} M[r][kk] X[kk][c], thread (r = tid / 16, h = tid % 16) taking kk = h, h + 16, ...; a batch
-// of terms' shared-memory reads before their products
-template <typename R>
-__device__ __forceinline__ void sb_acc_tile(const cpx<R> *Mt, const cpx<R> *X, cpx<R> (&acc)[SB_NR])
+// acc[i][c] += sum_{kk < 64} M[r][kk] X[kk][c], c < NR, for the warp's rows r = 2 w + i, lane h taking kk = h and h + 32:
+// the vector's entries, which are most of what a tile reads from shared memory, serve both rows. The reads of a term (in
+// complex64 of both) before their products. What bounds an updating CTA is these reads and FP32 products: with a row a
+// half warp (each entry read for one row) a tile of 8 columns took 147 KB of them against 82.
+template <typename R, int NR>
+__device__ __forceinline__ void sb_acc_tile(const cpx<R> *Mt, const cpx<R> *X, cpx<R> (&acc)[SB_RPW][NR])
 {
-    constexpr int XS = sb_xs<R>(), NK = SB_KT / SB_TPR;
-    const int r = threadIdx.x / SB_TPR, h = threadIdx.x % SB_TPR;
-    const cpx<R> *row = Mt + r * SB_TS;
+    constexpr int XS = sb_xs<R>(), NK = SB_KT / 32;
+    const int w = threadIdx.x >> 5, h = threadIdx.x & 31;
+    const cpx<R> *row = Mt + SB_RPW * w * SB_TS;
     if constexpr (sizeof(R) == 4) {
-        cpx<float> v[NK];
-        float4 y[NK][SB_NR / 2];
+        cpx<float> v[NK][SB_RPW];
+        float4 y[NK][NR / 2];
 #pragma unroll
         for (int u = 0; u < NK; ++u) {
-            const int kk = h + SB_TPR * u;
-            v[u] = row[kk];
+            const int kk = h + 32 * u;
+#pragma unroll
+            for (int i = 0; i < SB_RPW; ++i) v[u][i] = row[i * SB_TS + kk];
             const float4 *x = reinterpret_cast<const float4 *>(X + (size_t)kk * XS);
 #pragma unroll
-            for (int c2 = 0; c2 < SB_NR / 2; ++c2) y[u][c2] = x[c2];
+            for (int c2 = 0; c2 < NR / 2; ++c2) y[u][c2] = x[c2];
         }
 #pragma unroll
         for (int u = 0; u < NK; ++u)
 #pragma unroll
-            for (int c2 = 0; c2 < SB_NR / 2; ++c2) {
-                cfma<float>(acc[2 * c2], v[u], mk<float>(y[u][c2].x, y[u][c2].y));
-                cfma<float>(acc[2 * c2 + 1], v[u], mk<float>(y[u][c2].z, y[u][c2].w));
-            }
+            for (int c2 = 0; c2 < NR / 2; ++c2)
+#pragma unroll
+                for (int i = 0; i < SB_RPW; ++i) {
+                    cfma<float>(acc[i][2 * c2], v[u][i], mk<float>(y[u][c2].x, y[u][c2].y));
+                    cfma<float>(acc[i][2 * c2 + 1], v[u][i], mk<float>(y[u][c2].z, y[u][c2].w));
+                }
     } else {
-        constexpr int U = 2;
 #pragma unroll
-        for (int i0 = 0; i0 < NK; i0 += U) {
-            cpx<double> v[U];
-            double2 y[U][SB_NR];
+        for (int u = 0; u < NK; ++u) {
+            const int kk = h + 32 * u;
+            cpx<double> v[SB_RPW];
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int kk = h + SB_TPR * (i0 + u);
-                v[u] = row[kk];
-                const double2 *x = reinterpret_cast<const double2 *>(X + (size_t)kk * XS);
+            for (int i = 0; i < SB_RPW; ++i) v[i] = row[i * SB_TS + kk];
+            const double2 *x = reinterpret_cast<const double2 *>(X + (size_t)kk * XS);
 #pragma unroll
-                for (int c = 0; c < SB_NR; ++c) y[u][c] = x[c];
+            for (int c = 0; c < NR; ++c) {
+                const double2 y = x[c];
+#pragma unroll
+                for (int i = 0; i < SB_RPW; ++i) cfma<double>(acc[i][c], v[i], mk<double>(y.x, y.y));
             }
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-#pragma unroll
-                for (int c = 0; c < SB_NR; ++c) cfma<double>(acc[c], v[u], mk<double>(y[u][c].x, y[u][c].y));
         }
     }
 }
 
-// the 16 lanes of a chunk row: a halving exchange (4 + 2 + 1 values) leaves lane h with the sum of column h / 2
-// over 8 lanes, the last exchange adds its partner's (lanes h and h ^ 1 hold the same column)
 template <typename R>
-__device__ __forceinline__ cpx<R> sb_reduce_scatter(cpx<R> (&acc)[SB_NR])
+__device__ __forceinline__ cpx<R> sb_shfl_xor(cpx<R> v, int o)
 {
-    const int h = threadIdx.x % SB_TPR;
-    cpx<R> a4[4], a2[2];
-    const bool hi8 = h & 8, hi4 = h & 4, hi2 = h & 2;
+    return mk<R>(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+
+// the warp's 32 partial sums of its 2 NR values: halving exchanges (half the values to the partner, half kept) until a
+// lane has one, butterflies over the lanes that hold the same. Lane h ends with row h / 16, column (h % 16) NR / 16
+template <typename R, int N>
+__device__ __forceinline__ cpx<R> sb_halve(const cpx<R> (&a)[N], int o)
+{
+    if constexpr (N == 1) {
+        cpx<R> v = a[0];
+        for (; o; o >>= 1) v += sb_shfl_xor<R>(v, o);
+        return v;
+    } else {
+        const bool hi = threadIdx.x & o;
+        cpx<R> b[N / 2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const cpx<R> send = hi8 ? acc[j] : acc[j + 4], keep = hi8 ? acc[j + 4] : acc[j];
-        a4[j] = mk<R>(keep.x + __shfl_xor_sync(0xffffffffu, send.x, 8), keep.y + __shfl_xor_sync(0xffffffffu, send.y, 8));
+        for (int j = 0; j < N / 2; ++j) {
+            const cpx<R> send = hi ? a[j] : a[j + N / 2], keep = hi ? a[j + N / 2] : a[j];
+            b[j] = keep + sb_shfl_xor<R>(send, o);
+        }
+        return sb_halve<R, N / 2>(b, o >> 1);
     }
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const cpx<R> send = hi4 ? a4[j] : a4[j + 2], keep = hi4 ? a4[j + 2] : a4[j];
-        a2[j] = mk<R>(keep.x + __shfl_xor_sync(0xffffffffu, send.x, 4), keep.y + __shfl_xor_sync(0xffffffffu, send.y, 4));
-    }
-    const cpx<R> send = hi2 ? a2[0] : a2[1], keep = hi2 ? a2[1] : a2[0];
-    const cpx<R> a1 = mk<R>(keep.x + __shfl_xor_sync(0xffffffffu, send.x, 2), keep.y + __shfl_xor_sync(0xffffffffu, send.y, 2));
-    return mk<R>(a1.x + __shfl_xor_sync(0xffffffffu, a1.x, 1), a1.y + __shfl_xor_sync(0xffffffffu, a1.y, 1));
 }
 
 // waits (threads 0 .. cnt-1, one flag each) until flags[c0 ..] carry epoch; false (and M25_DEV_TIMEOUT) after about
@@ -339,7 +345,8 @@ __device__ __forceinline__ bool sb_wait_flags(const int *flags, int c0, int cnt,
 }
 
 // NBUF: tiles in the ring; TPB: tiles a product waits for at once (1, or a whole task of 4 with NBUF = 8)
-template <typename R, int NBUF, int TPB>
+// NR: columns computed (2, 4 or 8: the smallest that takes the right-hand sides)
+template <typename R, int NBUF, int TPB, int NR>
 __global__ void __launch_bounds__(SB_NT, 1) k_trsv_sb(SbSolve<R> a)
 {
     static_assert(SB_KTS % TPB == 0 && NBUF >= 2 * TPB, "whole batches, one in flight beside the one in use");
@@ -544,12 +551,14 @@ __global__ void __launch_bounds__(SB_NT, 1) k_trsv_sb(SbSolve<R> a)
             } else {
                 const int q = q_of_pos(s + 3), c0 = q * SB_CPB, cnt = min(SB_CPB, nch - c0);
                 if (!sb_wait_flags(a.tflag, c0, cnt, epoch, a.err, &ok)) { sb_wait_group<0>(); return; }
-                stage(a.Tx, SB_NR, SB_NR, q * SB);
+                stage(a.Tx, SB_NR, NR, q * SB);
             }
         }
-        C acc[SB_NR];
+        C acc[SB_RPW][NR];
 #pragma unroll
-        for (int j = 0; j < SB_NR; ++j) acc[j] = mk<R>(0, 0);
+        for (int i = 0; i < SB_RPW; ++i)
+#pragma unroll
+            for (int j = 0; j < NR; ++j) acc[i][j] = mk<R>(0, 0);
         for (int kt0 = 0; kt0 < SB_KTS; kt0 += TPB) {
 #pragma unroll
             for (int i = 0; i < TPB; ++i) issue();
@@ -557,14 +566,21 @@ __global__ void __launch_bounds__(SB_NT, 1) k_trsv_sb(SbSolve<R> a)
             __syncthreads();
 #pragma unroll
             for (int i = 0; i < TPB; ++i) {
-                sb_acc_tile<R>(tiles + (size_t)(used % NBUF) * SBC * SB_TS, Xs + (size_t)(kt0 + i) * SB_KT * XS, acc);
+                sb_acc_tile<R, NR>(tiles + (size_t)(used % NBUF) * SBC * SB_TS, Xs + (size_t)(kt0 + i) * SB_KT * XS, acc);
                 ++used;
             }
             __syncthreads();                                          // (the buffers are the next copies')
         }
-        const C v = sb_reduce_scatter<R>(acc);
-        if (!(tid & 1)) {                                             // lanes h, h ^ 1 hold column h / 2
-            C *sl = slots + (size_t)slot_of(k) * SBC * SB_NR + (tid / SB_TPR) * SB_NR + (tid % SB_TPR) / 2;
+        C flat[SB_RPW * NR];
+#pragma unroll
+        for (int i = 0; i < SB_RPW; ++i)
+#pragma unroll
+            for (int j = 0; j < NR; ++j) flat[i * NR + j] = acc[i][j];
+        const C v = sb_halve<R, SB_RPW * NR>(flat, 16);
+        const int lane = tid & 31;
+        if (!(lane & (16 / NR - 1))) {                                // one lane of those that hold the value
+            C *sl = slots + (size_t)slot_of(k) * SBC * SB_NR + (SB_RPW * (tid >> 5) + (lane >> 4)) * SB_NR +
+                    (lane & 15) * NR / 16;
             if (ph == 4) *sl = v;
             else *sl -= v;
         }
@@ -681,9 +697,14 @@ static int sb_solve_impl(const cpx<R> *A, long lda, int n, unsigned char *sb, co
     while (nbuf > 3 && sb_smem<R>(nbuf) > (size_t)optin) nbuf = nbuf == 8 ? 5 : 3;
     const size_t sm = sb_smem<R>(nbuf);
     M25_REQUIRE(sm <= (size_t)optin, "m25_sb_solve: shared memory");
-    const void *kf = batch4 ? (const void *)k_trsv_sb<R, 8, 4>
-                   : nbuf == 8 ? (const void *)k_trsv_sb<R, 8, 1> : nbuf == 5 ? (const void *)k_trsv_sb<R, 5, 1>
-                                                                         : (const void *)k_trsv_sb<R, 3, 1>;
+    auto of_nr = [&](auto nr) -> const void * {
+        constexpr int NR = decltype(nr)::value;
+        return batch4 ? (const void *)k_trsv_sb<R, 8, 4, NR>
+               : nbuf == 8 ? (const void *)k_trsv_sb<R, 8, 1, NR> : nbuf == 5 ? (const void *)k_trsv_sb<R, 5, 1, NR>
+                                                                                : (const void *)k_trsv_sb<R, 3, 1, NR>;
+    };
+    const void *kf = nrhs <= 2 ? of_nr(std::integral_constant<int, 2>()) : nrhs <= 4 ? of_nr(std::integral_constant<int, 4>())
+                                                                          : of_nr(std::integral_constant<int, 8>());
     M25_CHECK(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     void *kargs[] = {&args};
     M25_CHECK(cudaLaunchCooperativeKernel(kf, dim3(G), dim3(SB_NT), kargs, sm, s));
