@@ -3,6 +3,8 @@
 // the not-a-knot cubic spline to the fine uniform grid the fill interpolates, and the via kernels' spectra.
 // Restates multilayer.py:183-318 and via.py:36-235 (cited per kernel); complex128 throughout.
 #include <algorithm>
+#include <cooperative_groups.h>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -207,19 +209,17 @@ __global__ void k_via_spectra(const double *kr_, int npts, double w, Stack st, V
         zd Vh = voltage(st, nh, lo, hi), Ve = voltage(st, ne, lo, hi);
         return zdiv(jw * (Ve - Vh), kr * kr);
     };
-    int row = 0;
-    for (int r = 0; r < rq.nd; ++r, ++row) {                 // via.py:205-210
-        int kk = rq.dk[r], kb = rq.dspan[r][0], kt = rq.dspan[r][1];
-        zd spec = mk<double>(0, 0);
+    const int row = blockIdx.y;                              // one spectrum a row of the grid
+    zd spec = mk<double>(0, 0);
+    if (row < rq.nd) {                                       // via.py:205-210
+        int kk = rq.dk[row], kb = rq.dspan[row][0], kt = rq.dspan[row][1];
         for (int j = kb + 1; j <= kt; ++j) spec += zdiv(dV(j, kk), kz2[j]);
         spec = spec - zdiv(gq(kk, kb) * 1.0, jw);
         spec = spec + zdiv(gq(kk, kt), jw);
-        stc<double>(out, (size_t)row * npts + k, spec);
-    }
-    zd kr2 = kr * kr;
-    for (int r = 0; r < rq.nr; ++r, ++row) {                 // via.py:215-220 (P without the homogeneous term)
+    } else {                                                 // via.py:215-220 (P without the homogeneous term)
+        const int r = row - rq.nd;
+        zd kr2 = kr * kr;
         int mb = rq.rm[r][0], mt = rq.rm[r][1], nb = rq.rn[r][0], nt = rq.rn[r][1];
-        zd spec = mk<double>(0, 0);
         for (int i = mb + 1; i <= mt; ++i)
             for (int j = nb + 1; j <= nt; ++j)
                 spec += zdiv(kr2, kz2[i] * kz2[j]) * (dV(i, j) - dV(i, j - 1));
@@ -228,8 +228,8 @@ __global__ void k_via_spectra(const double *kr_, int npts, double w, Stack st, V
         for (int a = 0; a < 2; ++a)
             for (int b = 0; b < 2; ++b)
                 spec = spec - zdiv(gq(ka[a], kb2[b]) * (da[a] * da[b]), jw);
-        stc<double>(out, (size_t)row * npts + k, spec);
     }
+    stc<double>(out, (size_t)row * npts + k, spec);
 }
 
 // ---- complex Bessel J_n (mom25d_core.cpp:1510-1543: power series to |z| = 14, Hankel's expansion beyond) -------------
@@ -331,20 +331,22 @@ __global__ void k_via_homog(const double *rho, int n, double w, Stack st, unsign
 }
 
 // ---- Hankel transform (via.py:90-108): out[s, i] = (1/2pi) sum_k J0(rho_i kr_k) W[s, k] kr_k dk_k -------------------
-// One block per radius; the contour split over the threads (J0 of a real argument: the CUDA math library's j0;
-// on the lifted part the complex series above); then a block reduction per spectrum.
+// A cluster of HB blocks a radius: the contour split over their threads (J0 of a real argument: the CUDA math library's
+// j0; on the lifted part the complex series above), a block reduction per spectrum, then the blocks' sums added in
+// order through distributed shared memory. Bound by the FP64 Bessel values. HB = 4 where the radii alone do not fill
+// the SMs (a via group's distances, 1 to 64: 51 -> 20 us a launch), 1 where they do (the tables' 260 and 200: 88 us,
+// with 4 blocks 100).
 // RAW: the bare sum over real kr (hankel_real, mom25d_core.cpp:1430-1454): out[s, i] = sum_k J0(rho_i kr_k) W[s, k],
 // kr_ real f64[npts], no dk, no 1 / 2 pi.
-template <int NS, bool RAW = false>
-__global__ void __launch_bounds__(256) k_hankel(const double *kr_, const double *dk_, int npts, const double *W, int ns,
-                                                const double *rho, double *out, int nr)
+template <int NS, int HB, bool RAW = false>
+__global__ void __cluster_dims__(1, HB, 1) __launch_bounds__(256)
+k_hankel(const double *kr_, const double *dk_, int npts, const double *W, int ns, const double *rho, double *out, int nr)
 {
-    const int i = blockIdx.x;
-    if (i >= nr) return;
+    const int i = blockIdx.x;                              // (gridDim.x = nr)
     const double r = rho[i];
     zd acc[NS];
     for (int s = 0; s < NS; ++s) acc[s] = mk<double>(0, 0);
-    for (int k = threadIdx.x; k < npts; k += blockDim.x) {
+    for (int k = blockIdx.y * blockDim.x + threadIdx.x; k < npts; k += HB * blockDim.x) {
         zd f;
         if (RAW) {
             f = mk<double>(j0(r * kr_[k]), 0);
@@ -357,6 +359,7 @@ __global__ void __launch_bounds__(256) k_hankel(const double *kr_, const double 
             if (s < ns) acc[s] += f * ldc<double>(W, (size_t)s * npts + k);
     }
     __shared__ zd red[256 / 32][NS];
+    __shared__ zd part[NS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int s = 0; s < NS; ++s) {
         double x = acc[s].x, y = acc[s].y;
@@ -364,11 +367,20 @@ __global__ void __launch_bounds__(256) k_hankel(const double *kr_, const double 
         if (lane == 0) red[wid][s] = mk<double>(x, y);
     }
     __syncthreads();
-    if (threadIdx.x < NS && threadIdx.x < ns) {
+    if (threadIdx.x < NS) {
         zd t = mk<double>(0, 0);
         for (int j = 0; j < (int)(blockDim.x / 32); ++j) t += red[j][threadIdx.x];
+        part[threadIdx.x] = t;
+    }
+    if constexpr (HB > 1) cooperative_groups::this_cluster().sync();
+    else __syncthreads();
+    if (blockIdx.y == 0 && threadIdx.x < NS && threadIdx.x < ns) {
+        zd t = part[threadIdx.x];
+        if constexpr (HB > 1)
+            for (int q = 1; q < HB; ++q) t += *cooperative_groups::this_cluster().map_shared_rank(&part[threadIdx.x], q);
         stc<double>(out, (size_t)threadIdx.x * nr + i, RAW ? t : t * (1.0 / (2 * 3.14159265358979323846)));
     }
+    if constexpr (HB > 1) cooperative_groups::this_cluster().sync();   // (none leaves while another may read its sums)
 }
 
 // ---- not-a-knot cubic spline to a uniform grid (via.py:111-123; SciPy CubicSpline and PPoly evaluation) ------------
@@ -535,7 +547,7 @@ extern "C" int m25_spectral(const double *d_kr, int npts, double w, int nl, cons
     PairSpec *d_ps;
     M25_CHECK(cudaMallocAsync(&d_ps, sizeof(PairSpec) * (npair ? npair : 1), S(stream)));
     M25_CHECK(cudaMemcpyAsync(d_ps, ps, sizeof(PairSpec) * npair, cudaMemcpyHostToDevice, S(stream)));
-    k_spectral_tables<<<(npts + 127) / 128, 128, 0, S(stream)>>>(d_kr, npts, w, st, d_ps, npair, d_GA, d_GQ);
+    k_spectral_tables<<<(npts + 31) / 32, 32, 0, S(stream)>>>(d_kr, npts, w, st, d_ps, npair, d_GA, d_GQ);
     cudaError_t le = cudaGetLastError();
     cudaError_t fe = cudaFreeAsync(d_ps, S(stream));
     if (le != cudaSuccess) return m25_cuda_status(le, "k_spectral_tables");
@@ -568,7 +580,7 @@ extern "C" int m25_spectral_extracted(const double *d_kr, int npts, double w, in
     }
     M25_CHECK(cudaMemcpyAsync(d_pairs_scratch, ps, sizeof(PairSpec) * npair, cudaMemcpyHostToDevice, S(stream)));
     M25_CHECK(cudaStreamSynchronize(S(stream)));      // ps is a stack buffer: the copy must land first
-    k_spectral_tables<<<(npts + 127) / 128, 128, 0, S(stream)>>>(d_kr, npts, w, st, (const PairSpec *)d_pairs_scratch,
+    k_spectral_tables<<<(npts + 31) / 32, 32, 0, S(stream)>>>(d_kr, npts, w, st, (const PairSpec *)d_pairs_scratch,
                                                                  npair, d_GA, d_GQ);
     M25_LAUNCH_CHECK("k_spectral_tables");
     return M25_OK;
@@ -603,7 +615,10 @@ extern "C" int m25_via_spectra(const double *d_kr, int npts, double w, int nl, c
         rq.rm[i][0] = h_rm[2 * i]; rq.rm[i][1] = h_rm[2 * i + 1];
         rq.rn[i][0] = h_rn[2 * i]; rq.rn[i][1] = h_rn[2 * i + 1];
     }
-    k_via_spectra<<<(npts + 127) / 128, 128, 0, S(stream)>>>(d_kr, npts, w, st, rq, d_out);
+    if (nd + nr == 0) return M25_OK;
+    // a warp a block and a spectrum: a point's chain of complex divisions is what takes the time, so they go to as many
+    // SMs as there are (routed board, 13 spectra: 130 -> 110 us against a thread doing all 13, 128 a block)
+    k_via_spectra<<<dim3((npts + 31) / 32, nd + nr), 32, 0, S(stream)>>>(d_kr, npts, w, st, rq, d_out);
     M25_LAUNCH_CHECK("k_via_spectra");
     return M25_OK;
 }
@@ -620,14 +635,26 @@ extern "C" int m25_via_homog(const double *d_rho, int n, double w, int nl, const
     return M25_OK;
 }
 
+template <bool RAW>
+static void hankel_launch(const double *kr, const double *dk, int npts, const double *W, int ns, const double *rho,
+                          double *out, int nr, cudaStream_t s)
+{
+    auto go = [&](auto nsm) {
+        constexpr int NS = decltype(nsm)::value;
+        if (nr > 148) k_hankel<NS, 1, RAW><<<nr, 256, 0, s>>>(kr, dk, npts, W, ns, rho, out, nr);
+        else k_hankel<NS, 4, RAW><<<dim3(nr, 4), 256, 0, s>>>(kr, dk, npts, W, ns, rho, out, nr);
+    };
+    if (ns <= 4) go(std::integral_constant<int, 4>());
+    else if (ns <= 8) go(std::integral_constant<int, 8>());
+    else go(std::integral_constant<int, 16>());
+}
+
 extern "C" int m25_hankel(const double *d_kr, const double *d_dk, int npts, const double *d_W, int ns,
                           const double *d_rho, int nr, double *d_out, void *stream)
 {
     M25_REQUIRE(ns >= 1 && ns <= 16, "m25_hankel: 1 to 16 spectra a call");
     if (!nr) return M25_OK;
-    if (ns <= 4) k_hankel<4><<<nr, 256, 0, S(stream)>>>(d_kr, d_dk, npts, d_W, ns, d_rho, d_out, nr);
-    else if (ns <= 8) k_hankel<8><<<nr, 256, 0, S(stream)>>>(d_kr, d_dk, npts, d_W, ns, d_rho, d_out, nr);
-    else k_hankel<16><<<nr, 256, 0, S(stream)>>>(d_kr, d_dk, npts, d_W, ns, d_rho, d_out, nr);
+    hankel_launch<false>(d_kr, d_dk, npts, d_W, ns, d_rho, d_out, nr, S(stream));
     M25_LAUNCH_CHECK("k_hankel");
     return M25_OK;
 }
@@ -637,9 +664,7 @@ extern "C" int m25_hankel_real(const double *d_rho, int nr, const double *d_kr, 
 {
     M25_REQUIRE(ns >= 1 && ns <= 16, "m25_hankel_real: 1 to 16 rows of W a call");
     if (!nr) return M25_OK;
-    if (ns <= 4) k_hankel<4, true><<<nr, 256, 0, S(stream)>>>(d_kr, nullptr, nk, d_W, ns, d_rho, d_out, nr);
-    else if (ns <= 8) k_hankel<8, true><<<nr, 256, 0, S(stream)>>>(d_kr, nullptr, nk, d_W, ns, d_rho, d_out, nr);
-    else k_hankel<16, true><<<nr, 256, 0, S(stream)>>>(d_kr, nullptr, nk, d_W, ns, d_rho, d_out, nr);
+    hankel_launch<true>(d_kr, nullptr, nk, d_W, ns, d_rho, d_out, nr, S(stream));
     M25_LAUNCH_CHECK("k_hankel");
     return M25_OK;
 }
