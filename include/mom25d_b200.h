@@ -82,6 +82,11 @@ int m25_device_info(int *sm_count, size_t *free_bytes, size_t *total_bytes);
 int m25_spectral(const double *d_kr, int npts, double w, int nl, const double *h_h, const double *h_eps,
                  int top_open, const double *h_top_eps, int npair, const int *h_o, const int *h_s,
                  double *d_GA, double *d_GQ, void *stream);
+/* The nodes kr and weights dk of the Sommerfeld contour (via.py:36-53): nq-point Gauss-Legendre (h_x, h_w on [-1, 1],
+ * nq <= 16) on m1 equal pieces of [0, t1], lifted into the upper half plane by alpha sin(pi t / t1), then on n2 pieces
+ * of width wid2 of the real axis from t1, the last ending at K. kr, dk complex128[(m1 + n2) * nq]. */
+int m25_contour(double t1, double alpha, double K, double wid2, int m1, int n2, const double *h_x, const double *h_w,
+                int nq, double *d_kr, double *d_dk, void *stream);
 /* out[s, i] = (1/2pi) sum_k J0(rho_i kr_k) W[s, k] kr_k dk_k over a contour whose first nlift points are complex
  * (replaces via.py:104-108 hankel, with mom25d_core.cpp:1430-1454 hankel_real and :1510-1558 bessel_jn_complex).
  * kr, dk complex128[npts]; W complex128[ns*npts]; rho f64[nr]; out complex128[ns*nr]. */

@@ -24,18 +24,26 @@ VIA_NRHO = 200                                                # via.py:179
 VIA_TABLE_PAIRS = 64                                          # sim.py:784
 
 
-def sommerfeld_contour(f, st, rho_max, K=None, nq=8):
-    """Nodes and weights of the Sommerfeld integration path (via.py:36-53): lifted into the upper half plane by
-    alpha sin up to 1.5 k_max, then real to K; Gauss-Legendre (nq points) on each piece."""
+GAUSS = {nq: np.polynomial.legendre.leggauss(nq) for nq in (8,)}        # the contour's rule
+
+
+def contour_path(f, st, rho_max, K=None):
+    """The pieces of the Sommerfeld integration path (via.py:36-53): lifted into the upper half plane by alpha sin up to
+    t1 = 1.5 k_max in m1 equal pieces, then real to K in pieces of wid2, n2 of them: (t1, alpha, K, wid2, m1, n2)."""
     k0 = 2 * np.pi * f / C0
     kmax = k0 * np.sqrt(st.max_er())
     K = K or (max(1e5, 30.0 / st.hmin) + 40 * kmax)
     t1, alpha = 1.5 * kmax, min(0.5 * k0, 4.0 / rho_max)
     wid1, wid2 = min(0.3 * k0, 0.8 * alpha), 2 * np.pi / rho_max
-    b1 = np.linspace(0, t1, int(np.ceil(t1 / wid1)) + 1)
-    b2 = np.append(np.arange(t1, K, wid2), K)
-    br = np.concatenate([b1, b2[1:]])
-    xg, wg = np.polynomial.legendre.leggauss(nq)
+    return t1, alpha, K, wid2, int(np.ceil(t1 / wid1)), int(np.ceil((K - t1) / wid2))
+
+
+def sommerfeld_contour(f, st, rho_max, K=None, nq=8):
+    """Nodes and weights on the path's pieces, Gauss-Legendre (nq points) on each, on the host (the device's are
+    m25_contour's)."""
+    t1, alpha, K, wid2, m1, n2 = contour_path(f, st, rho_max, K)
+    xg, wg = GAUSS[nq] if nq in GAUSS else np.polynomial.legendre.leggauss(nq)
+    br = np.concatenate([np.linspace(0, t1, m1 + 1), t1 + wid2 * np.arange(1, n2), [K]])
     a, b = br[:-1, None], br[1:, None]
     t = (0.5 * (b - a) * xg[None, :] + 0.5 * (a + b)).ravel()
     wt = (0.5 * (b - a) * wg[None, :]).ravel()
@@ -56,6 +64,19 @@ class _StackArgs:
 
     def args(self):
         return (c_int(self.nl), P(self.h), P(self.eps), c_int(self.top_open), P(self.top_eps))
+
+
+def _upload(*arrays):
+    """Host arrays (complex128, float64, int32) as device tensors, in one copy: views of one buffer, each on a 16-byte
+    boundary."""
+    raw = [np.ascontiguousarray(a).reshape(-1).view(np.uint8) for a in arrays]
+    at = np.cumsum([0] + [(r.size + 15) // 16 * 16 for r in raw])
+    host = np.zeros(at[-1], np.uint8)
+    for o, r in zip(at, raw):
+        host[o:o + r.size] = r
+    dev = torch.from_numpy(host).to('cuda')
+    kinds = {np.dtype(complex): torch.complex128, np.dtype(float): torch.float64, np.dtype(np.int32): torch.int32}
+    return [dev[o:o + r.size].view(kinds[np.asarray(a).dtype]) for a, o, r in zip(arrays, at, raw)]
 
 
 class DeviceGeometry:
@@ -171,15 +192,14 @@ class DeviceTables:
                 dimg[i] = 2 * st.nearest_discontinuity(a)
                 ext.append((i, 'i', 18.0 / dimg[i], 2 * np.pi))
         if ext:
-            kr = _lib.dev(np.array([e[2] for e in ext], complex))
-            ww = _lib.dev(np.array([e[3] for e in ext], float))
-            ga = torch.empty(len(ext), dtype=torch.complex128, device='cuda')
-            gq = torch.empty_like(ga)
+            kr, ww = _upload(np.array([e[2] for e in ext], complex), np.array([e[3] for e in ext], float))
+            gg = torch.empty((2, len(ext)), dtype=torch.complex128, device='cuda')
+            ga, gq = gg
             for j, (i, kind, K1, wj) in enumerate(ext):
                 a, b = pairs[i][0], pairs[i][1]
                 check(lib().m25_spectral_points(P(kr[j:]), P(ww[j:]), c_int(1), *dg.stack.args(), c_int(a), c_int(b),
                                                 P(ga[j:]), P(gq[j:]), s), 'm25_spectral_points')
-            ga, gq = ga.cpu().numpy(), gq.cpu().numpy()
+            ga, gq = gg.cpu().numpy()
             for j, (i, kind, K1, wj) in enumerate(ext):
                 a = pairs[i][0]
                 if kind == 'x':
@@ -199,9 +219,17 @@ class DeviceTables:
             for j, (x, y, z) in enumerate(lst):
                 ed[i, j], ecA[i, j], ecq[i, j] = x, y, z
         # the contour and the spectra with the extracted parts removed
-        krh, dkh, K = sommerfeld_contour(f, st, geo.rho_max)
-        self.npts = npts = len(krh)
-        d_kr, d_dk = _lib.dev(krh), _lib.dev(dkh)
+        xg, wg = GAUSS[8]
+        t1, alpha, K, wid2, m1, n2 = contour_path(f, st, geo.rho_max)
+        self.npts = npts = (m1 + n2) * len(xg)
+        d_kr, d_dk = torch.empty((2, npts), dtype=torch.complex128, device='cuda')
+        check(lib().m25_contour(c_double(t1), c_double(alpha), c_double(K), c_double(wid2), c_int(m1), c_int(n2), P(xg),
+                                P(wg), c_int(len(xg)), P(d_kr), P(d_dk), s), 'm25_contour')
+        rho_max = geo.rho_max
+        nf = TABLE_NFINE
+        dx = np.linspace(0, rho_max, nf)[1]
+        self.scal, self.dr, self.d, self.dimg, self.kind = _upload(np.concatenate([cA, cq, cAi, cqi]),
+                                                                   np.full(npair, dx), dd, dimg, kind)
         W = torch.empty((2 * npair, npts), dtype=torch.complex128, device='cuda')   # GA rows, then GQ rows
         scratch = torch.empty(int(lib().m25_pair_record_bytes()), dtype=torch.uint8, device='cuda')
         h_o = np.array([p[0] for p in pairs], np.int32)      # (host arrays kept alive across the call)
@@ -217,22 +245,14 @@ class DeviceTables:
             check(lib().m25_hankel(P(d_kr), P(d_dk), c_int(npts), P(W[r0:]), c_int(r1 - r0), P(dg.d_rho),
                                    c_int(TABLE_NRHO), P(H[r0:]), s), 'm25_hankel')
         self.H = H
-        rho_max = geo.rho_max
-        nf = TABLE_NFINE
-        dx = np.linspace(0, rho_max, nf)[1]
         self.AQ = torch.empty((2 * npair, nf), dtype=torch.complex128, device='cuda')
         check(lib().m25_spline_uniform(P(dg.d_rho), P(H), c_int(2 * npair), c_int(TABLE_NRHO), c_double(dx), c_int(nf),
                                        P(self.AQ), c_int(0), c_long(nf), c_long(0), c_int(1), s), 'm25_spline_uniform')
-        self.scal = _lib.dev(np.concatenate([cA, cq, cAi, cqi]))
-        self.dr = _lib.dev(np.full(npair, dx))
-        self.d = _lib.dev(dd)
-        self.dimg = _lib.dev(dimg)
-        self.kind = _lib.dev(kind)
         self.host = dict(cA=cA, cq=cq, cAi=cAi, cqi=cqi, d=dd, dimg=dimg, kind=kind, dr=np.full(npair, dx))
         self.tables = _lib.Tables(npair, nf, len(geo.layers), P(self.AQ), P(self.AQ[npair:]), P(self.scal),
                                   P(self.scal[npair:]), P(self.scal[2 * npair:]), P(self.scal[3 * npair:]),
                                   P(self.dr), P(self.d), P(self.dimg), P(dg.tab), P(self.kind))
-        self.kr, self.dk, self.d_kr, self.d_dk = krh, dkh, d_kr, d_dk
+        self.d_kr, self.d_dk = d_kr, d_dk
         self.tables32 = None
         if single:
             nf32 = TABLE_NFINE32

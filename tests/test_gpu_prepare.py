@@ -80,3 +80,27 @@ def test_spline(n):
     want = np.array([CubicSpline(x, r)(np.linspace(0, x[-1], nf)) for r in y])
     # both solve the system to rounding: differences of a few hundred ulp of the largest sample (steep end pieces)
     assert np.abs(out.cpu().numpy() - want).max() <= 1e-12
+
+
+@pytest.mark.parametrize('f', [0.1e9, 1.0e9, 4.0e9, 10.0e9])
+@pytest.mark.parametrize('board', ['microstrip', 'stub'])
+def test_contour(board, f):
+    """The device's contour against the host's: the same pieces, nodes and weights to rounding."""
+    from mom25d_b200 import _lib, board as B, device
+    from mom25d_b200._lib import P, check, lib
+    bd = B.microstrip_board(dmax=0.6e-3, length=10e-3) if board == 'microstrip' else B.stub_filter_board(dmax=0.3e-3)
+    rho_max = float(np.ptp(bd.nodes[:, 0]) + np.ptp(bd.nodes[:, 1]))
+    kr, dk, K = device.sommerfeld_contour(f, bd.stack, rho_max)
+    t1, alpha, K2, wid2, m1, n2 = device.contour_path(f, bd.stack, rho_max)
+    assert K2 == K and (m1 + n2) * 8 == len(kr)
+    xg, wg = device.GAUSS[8]
+    out = torch.empty((2, len(kr)), dtype=torch.complex128, device='cuda')
+    D = ctypes.c_double
+    check(lib().m25_contour(D(t1), D(alpha), D(K), D(wid2), m1, n2, P(xg), P(wg), 8, P(out[0]), P(out[1]),
+                            _lib.stream_ptr()), 'm25_contour')
+    _lib.sync_check()
+    got = out.cpu().numpy()
+    # breakpoints of up to K = m1 + n2 steps: a few ulp of K in a node, relative to a piece's width in a weight
+    assert np.abs(got[0] - kr).max() <= 8 * 2.0 ** -53 * K
+    assert np.abs(got[1] - dk).max() <= 16 * 2.0 ** -53 * K
+    assert np.array_equal(got[0].imag == 0, kr.imag == 0)
