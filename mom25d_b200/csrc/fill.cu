@@ -73,10 +73,13 @@ __device__ __forceinline__ R cdist2(const double *c, int p, int q)
 // transposed through shared memory (0.5 evaluations an entry). On the diagonal tiles an entry below the diagonal is
 // formed as its mirror image is, so Z is exactly symmetric there too. A tile whose distinct pairs do not fit the
 // shared-memory budget evaluates its entries directly.
-// Bound by FP64 instructions and the tables' gathers (about 96 bytes of L2 sectors an evaluation). Ne = 8,508: 2.22 ms
-// with every tile computed, divisions by r and 4 complex products an entry, 1.44 ms so; Ne = 18,763: 11.0 -> 6.9 ms
-// (5.6 GB written: 0.85 ms).
-struct EdgeHalves { int p[2]; int lt[2]; double a[2], ax[2], ay[2]; };    // a = +-l / 2A x A; a times (centroid - vertex)
+// Bound by shared-memory reads and the tables' gathers (about 96 bytes of L2 sectors an evaluation). Ne = 8,508: 2.22 ms
+// with every tile computed, divisions by r and 4 complex products an entry, 1.01 ms now; Ne = 18,763: 11.0 ms then (5.6
+// GB written: 0.85 ms).
+// The halves of a tile's 32 row (or column) edges: triangle, its layer; a = +-l / 2A x A; a times (centroid - vertex). By
+// half, then edge: a lane's column edge is read without bank conflicts (as an array of 64-byte structs, sixteen lanes to
+// a bank, these reads were 84% of the shared-memory cycles and the fill's bound: 1.44 ms at Ne = 8,508).
+struct EdgeHalves { int p[2][32], lt[2][32]; double a[2][32], ax[2][32], ay[2][32]; };
 
 #define FF_SMEM (48 * 1024)
 
@@ -99,7 +102,7 @@ __device__ __forceinline__ void fill_far_tile(R *Z, long ld, const m25_mesh &g, 
     constexpr int GCAP = FF_SMEM / (2 * sizeof(C));                   // distinct triangle pairs a tile holds
     C *gas = reinterpret_cast<C *>(ff_raw), *gqs = gas + GCAP;
     static_assert(32 * 33 * sizeof(C) <= FF_SMEM, "the transposed tile in the pairs' memory");
-    __shared__ EdgeHalves rows[32], cols[32];
+    __shared__ EdgeHalves E[2];                                       // row edges, column edges
     __shared__ short uid[2][64];                                      // [row / col][edge half 2 e + s] -> distinct index
     __shared__ int tri[2][64];                                        // distinct triangles, in first-seen order
     __shared__ unsigned rep_mask[2][2];
@@ -108,30 +111,32 @@ __device__ __forceinline__ void fill_far_tile(R *Z, long ld, const m25_mesh &g, 
     upper_tile(blockIdx.x, (g.Ne + 31) / 32, by, bx);
     const int M0 = by * 32, N0 = bx * 32;
     const int lane = threadIdx.x, wid = threadIdx.y, tid = wid * 32 + lane;
-    if (tid < 64) {
-        int e = (tid < 32 ? M0 : N0) + (tid & 31);
-        EdgeHalves h;
+    if (tid < 128) {                                                  // a thread a half: side, half, edge
+        EdgeHalves &h = E[tid >> 6];
+        const int hf = (tid >> 5) & 1, j = tid & 31, e = (tid < 64 ? M0 : N0) + j;
+        int p = 0, lt = 0;
+        double al = 0, ax = 0, ay = 0;
         if (e < g.Ne) {
-            int pp = g.ep[e], pm = g.em[e];
-            h.p[0] = pp; h.p[1] = pm;
-            h.lt[0] = g.lt[pp]; h.lt[1] = g.lt[pm];
-            h.a[0] = g.ap[e] * g.area[pp]; h.a[1] = g.am[e] * g.area[pm];
-            h.ax[0] = h.a[0] * (g.cent[2 * pp] - g.vp[2 * e]); h.ay[0] = h.a[0] * (g.cent[2 * pp + 1] - g.vp[2 * e + 1]);
-            h.ax[1] = h.a[1] * (g.cent[2 * pm] - g.vm[2 * e]); h.ay[1] = h.a[1] * (g.cent[2 * pm + 1] - g.vm[2 * e + 1]);
-        } else {
-            h.p[0] = h.p[1] = 0; h.lt[0] = h.lt[1] = 0; h.a[0] = h.a[1] = 0; h.ax[0] = h.ax[1] = h.ay[0] = h.ay[1] = 0;
+            p = hf ? g.em[e] : g.ep[e];
+            lt = g.lt[p];
+            const double *v = hf ? g.vm : g.vp;
+            al = (hf ? g.am[e] : g.ap[e]) * g.area[p];
+            ax = al * (g.cent[2 * p] - v[2 * e]);
+            ay = al * (g.cent[2 * p + 1] - v[2 * e + 1]);
         }
-        (tid < 32 ? rows : cols)[tid & 31] = h;
+        h.p[hf][j] = p; h.lt[hf][j] = lt;
+        h.a[hf][j] = al; h.ax[hf][j] = ax; h.ay[hf][j] = ay;
     }
     __syncthreads();
     // distinct triangles of the row halves (threads 0 .. 63) and of the column halves (64 .. 127): a half is its
     // triangle's representative when no earlier half has the triangle; representatives are numbered by a ballot
     int side = tid >> 6, hh = tid & 63, first = -1, x = -1;
     if (tid < 128) {
-        const EdgeHalves *E = side ? cols : rows;
-        x = E[hh >> 1].p[hh & 1];
-        for (int j = 0; j < hh; ++j)
-            if (E[j >> 1].p[j & 1] == x) { first = j; break; }
+        const EdgeHalves &h = E[side];
+        x = h.p[hh & 1][hh >> 1];
+#pragma unroll 8
+        for (int j = 63; j >= 0; --j)                      // (the earliest; no branch, so the reads overlap)
+            if (j < hh && h.p[j & 1][j >> 1] == x) first = j;
         const unsigned m = __ballot_sync(0xffffffffu, first < 0);
         if ((tid & 31) == 0) rep_mask[side][(tid >> 5) & 1] = m;
     }
@@ -163,12 +168,11 @@ __device__ __forceinline__ void fill_far_tile(R *Z, long ld, const m25_mesh &g, 
     __syncthreads();
     const int n = N0 + lane;
     const R wr = (R)w, qw = (R)(4.0 / w);
-    const EdgeHalves &B = cols[lane];
+    const EdgeHalves &A = E[0], &B = E[1];
     C val[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int i = wid + 8 * k, m = M0 + i;
-        const EdgeHalves &A = rows[i];
         const bool up = m <= n;                           // else the terms in the mirror image's order
         C sa = mk<R>(0, 0), sq = mk<R>(0, 0);
 #pragma unroll
@@ -182,9 +186,10 @@ __device__ __forceinline__ void fill_far_tile(R *Z, long ld, const m25_mesh &g, 
                     ga = gas[q];
                     gq = gqs[q];
                 } else {
-                    tab_kern<R>(tb, A.lt[s], B.lt[t], cdist2<R>(g.cent, A.p[s], B.p[t]), ga, gq);
+                    tab_kern<R>(tb, A.lt[s][i], B.lt[t][lane], cdist2<R>(g.cent, A.p[s][i], B.p[t][lane]), ga, gq);
                 }
-                const R c = (R)A.ax[s] * (R)B.ax[t] + (R)A.ay[s] * (R)B.ay[t], q = (R)A.a[s] * (R)B.a[t];
+                const R c = (R)A.ax[s][i] * (R)B.ax[t][lane] + (R)A.ay[s][i] * (R)B.ay[t][lane];
+                const R q = (R)A.a[s][i] * (R)B.a[t][lane];
                 sa.x = fma(c, ga.x, sa.x); sa.y = fma(c, ga.y, sa.y);
                 sq.x = fma(q, gq.x, sq.x); sq.y = fma(q, gq.y, sq.y);
             }
