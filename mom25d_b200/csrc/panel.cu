@@ -6,11 +6,13 @@
 //     groups of GRP whose entries stay in the owner thread's registers: inside a group a column needs the pivot search,
 //     the GRP entries of two rows exchanged, and nothing from memory;
 //   - the exchange is by st.async into distributed shared memory, completion counted in bytes on the receiver's
-//     mbarriers: every CTA sends its candidate (value, row) to every CTA; the winner's CTA then sends its row and the
-//     pivot's reciprocal to all, the diagonal row's CTA that row to the winner's. While the candidates travel, the rows
-//     that may be sent are made ready and the other warps finish the column before (every 16-byte message costs the
-//     receiver an update of its mbarrier: sending every candidate's row along with it, one trip a column instead of
-//     two, took 1.05 to 1.2 times as long);
+//     mbarriers: every CTA sends its candidate's entry to every CTA; the winner's CTA then sends its row to all, the
+//     diagonal row's CTA that row to the winner's. While the candidates travel, the rows that may be sent are made ready
+//     and the other warps finish the column before; while the row travels, one warp forms the pivot's reciprocal. (Every
+//     16-byte message costs the receiver an update of its mbarrier: sending every candidate's row along with it, one
+//     trip a column instead of two, took 1.05 to 1.2 times as long.) What the warp of a CTA's candidate has to do in a
+//     column is what a column takes, so the reciprocal (in f64 390 cycles) and the bookkeeping of the interchanges are
+//     other warps' work (LUs 2 to 4% shorter at n = 2,000 to 6,000);
 //   - the searches are integer redux over the bit patterns of |re| + |im| (non-negative: ordered as integers);
 //   - at a group's end the group's interchanges are applied to the panel's other columns as one permutation and its
 //     GRP rows of U are solved (a warp a column), then every thread updates its rows of the columns to the right: those
@@ -20,9 +22,8 @@
 // in at the end), so one loop body serves every column of a group.
 // Every entry takes its terms a -= l u one at a time in column order, as an unblocked elimination does.
 //
-// 64 columns alone on the GPU, complex64: 111 us at 2,000 rows, 145 at 8,000, 227 at 16,000 (about 3,300 cycles a column
-// at 2,000); the panel kernel with its rows in shared memory (k_panel_smem) took 206-218 us inside LUs of 5,000 and
-// 9,601 in a cluster of 16 and 258-303 us on 32 cooperative CTAs.
+// 64 columns inside an LU: complex64 n = 4,977: 118 us, complex128 n = 2,921: 146 us; the panel kernel with its rows in
+// shared memory (k_panel_smem) took 206 and 292 us there in a cluster of 16 and 258 to 303 us on 32 cooperative CTAs.
 #include <algorithm>
 
 #include "common.cuh"
@@ -122,8 +123,10 @@ __device__ __forceinline__ uint4 piece_of(cpx<double> x, int)        // (an entr
 template <typename R, int GRP> struct PanelShared {
     typedef cpx<R> C;
     static constexpr int RB = GRP * (int)sizeof(C) / 16;              // 16-byte pieces of a row's GRP entries
-    uint4 head[2][PCL_MAX];                  // each CTA's candidate (value, row), by column parity
-    struct __align__(16) Row { C row[GRP]; uint4 rc; } win[2];        // the pivot row and 1 / pivot
+    uint4 head[2][PCL_MAX];                  // each CTA's candidate's entry (NaN: none), by column parity
+    struct __align__(16) Row { C row[GRP]; uint4 p; } win[2];         // the pivot row and its index
+    uint4 rcp[2];                            // 1 / pivot
+    int pos[32], src[32];                    // the group's interchanges (plan), for the other columns
     C diag[2][GRP];                          // the diagonal row, in the CTA of the pivot row
     struct __align__(16) Stage { C row[GRP]; C l, next; } stage[2];   // a row on its way out: candidate, diagonal row
     C prow[GRP][GRP];                        // the group's pivot rows (rotated as they were sent)
@@ -164,7 +167,7 @@ __global__ void __launch_bounds__(T, 1) k_panel_cluster(R *A, long lda, int n, i
     bool dead = false;                                     // (block-uniform) after a failure: barriers only, to the end
     for (int g0 = 0; g0 < jb; g0 += GRP) {
         const int gw = min(GRP, jb - g0), gr = k0 + g0;    // the group's columns and its first row / column
-        // the group's interchanges as a permutation, in each warp's lanes: row pos ends with what row src held. Lanes
+        // the group's interchanges as a permutation, in the last warp's lanes: row pos ends with what row src held. Lanes
         // 0 .. GRP - 1: the group's own rows; lane GRP + j: the row below that column j's interchange touched first
         int pos = lane < gw ? gr + lane : -1, src = pos, plast = -1;
         R best = (R)-1;
@@ -247,51 +250,75 @@ __global__ void __launch_bounds__(T, 1) k_panel_cluster(R *A, long lda, int n, i
             if (failed) { dead = true; break; }
             of_head(ch, best, bi);
             warp_best(best, bi);
-            // out to every CTA; the warp of its thread, and the warp of the diagonal row's thread, get the rows ready
+            // its entry out to every CTA; its thread's warp, and the warp of the diagonal row's thread, get the rows
+            // ready
             const int cw = bi == PNONE ? 0 : ((bi - r0) & (T - 1)) >> 5;
             const int dw = col >= r0 && col < rend ? ((col - r0) & (T - 1)) >> 5 : -1;
-            uint4 cp = make_uint4(0u, 0u, 0u, 0u), dp = cp, rcp = cp;
+            uint4 cp = make_uint4(0u, 0u, 0u, 0u), dp = cp;
             const bool busy = wid == cw || wid == dw;
-            if (wid == cw) {
-                if (G > 1 && lane < G)
-                    send16(peer_addr(smem_addr(&s.head[par][b]), lane), head_of(best, bi), peer_addr(hbar, lane));
-                C z;
-                cp = prepare(jj, bi, s.stage[0], z);
+            auto recip = [&](C z) -> uint4 {
                 C rc = mk<R>(0, 0);
                 if (!(z.x == 0 && z.y == 0)) rc = cdiv<R>(mk<R>(1, 0), z);
-                memcpy(&rcp, &rc, sizeof(C));
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                memcpy(&v, &rc, sizeof(C));
+                return v;
+            };
+            if (wid == cw) {
+                if (G > 1) {
+                    C z = mk<R>(0, 0);
+#pragma unroll
+                    for (int r = 0; r < RPT; ++r)
+                        if (r0 + tid + T * r == bi) z = jj == 0 ? a[r][0] : next[r];
+                    const int from = bi == PNONE ? 0 : (bi - r0) & 31;
+                    z = mk<R>(__shfl_sync(0xffffffffu, z.x, from), __shfl_sync(0xffffffffu, z.y, from));
+                    if (bi == PNONE) z.x = (R)NAN;
+                    uint4 h = make_uint4(0u, 0u, 0u, 0u);
+                    memcpy(&h, &z, sizeof(C));
+                    if (lane < G) send16(peer_addr(smem_addr(&s.head[par][b]), lane), h, peer_addr(hbar, lane));
+                }
+                C z;
+                cp = prepare(jj, bi, s.stage[0], z);
+                if (G == 1 && lane == 0) s.rcp[par] = recip(z);
             }
             if (wid == dw) {
                 C z;
                 dp = prepare(jj, col, s.stage[1], z);
             }
             if (jj > 0) {
-                plan(jj - 1);
+                if (wid == nw - 1) plan(jj - 1);
                 if (!busy) rest(jj - 1);
             }
-            // the winner
+            // the winner: the largest entry, of the first CTA on ties (the CTAs' rows are in order)
             bool ok = true;
-            int p = bi, wq = 0;
+            int wq = 0;
+            C piv = mk<R>(0, 0);
             if (G > 1) {
                 ok = wait_phase(hbar, phase, err);
-                R bv = (R)0;
-                int row = PNONE;
-                if (lane < G) of_head(s.head[par][lane], bv, row);
-                p = row;
-                warp_best(bv, p);
-                wq = __ffs(__ballot_sync(0xffffffffu, lane < G && row == p)) - 1;
+                if (lane < G) {
+                    const uint4 h = s.head[par][lane];
+                    memcpy(&piv, &h, sizeof(C));
+                }
+                R v = abs1(piv);
+                const bool is = lane < G && v == v;
+                int row = is ? lane : PNONE;
+                warp_best(v, row);
+                wq = row;
+            } else if (bi == PNONE) {
+                wq = PNONE;
             }
             if (!ok) dev_error(err, M25_DEV_TIMEOUT);
-            else if (p < col || p >= n) {                   // no candidate (NaN in the whole column): every CTA alike
+            else if (wq == PNONE) {                          // no candidate (NaN in the whole column): every CTA alike
                 if (tid == 0) dev_error(err, M25_DEV_INDEX);
                 ok = false;
             }
-            // its row and reciprocal to every CTA, the diagonal row to its CTA
+            // its row to every CTA, the diagonal row to its CTA; in each CTA a warp without a row forms 1 / pivot
             typename PS::Row &win = s.win[par];
             const int piece = lane & (RB - 1);
             if (ok) {
-                if (G > 1 && tid == 0) expect_bytes(rbar, (RB + 1 + (wq == b && p != col ? RB : 0)) * 16u);
-                if (wid == cw && wq == b) {
+                const bool own = wq == b, swap = !own || bi != col;
+                if (G > 1 && tid == 0) expect_bytes(rbar, (RB + 2 + (own && swap ? RB : 0)) * 16u);
+                if (own && wid == cw) {
+                    const uint4 pi = make_uint4((unsigned)bi, 0u, 0u, 0u);
                     if (G > 1) {
                         const uint32_t d = smem_addr(&win.row[0]) + 16 * piece;
 #pragma unroll
@@ -299,30 +326,37 @@ __global__ void __launch_bounds__(T, 1) k_panel_cluster(R *A, long lda, int n, i
                             const int q = lane / RB + 32 / RB * i;
                             if (q < G) send16(peer_addr(d, q), cp, peer_addr(rbar, q));
                         }
-                        if (lane < G) send16(peer_addr(smem_addr(&win.rc), lane), rcp, peer_addr(rbar, lane));
+                        if (lane < G) send16(peer_addr(smem_addr(&win.p), lane), pi, peer_addr(rbar, lane));
                     } else {
                         if (lane < RB) reinterpret_cast<uint4 *>(win.row)[lane] = cp;
-                        if (lane == 0) win.rc = rcp;
+                        if (lane == 0) win.p = pi;
                     }
                 }
-                if (wid == dw && p != col && lane < RB) {
+                if (wid == dw && swap && lane < RB) {
                     if (G > 1) send16(peer_addr(smem_addr(&s.diag[par][0]) + 16 * lane, wq), dp, peer_addr(rbar, wq));
                     else reinterpret_cast<uint4 *>(s.diag[par])[lane] = dp;
+                }
+                const int helper = cw != 0 && dw != 0 ? 0 : cw != 1 && dw != 1 ? 1 : 2;
+                if (G > 1 && wid == helper) {
+                    const C z = mk<R>(__shfl_sync(0xffffffffu, piv.x, wq), __shfl_sync(0xffffffffu, piv.y, wq));
+                    const uint4 v = recip(z);
+                    if (lane == 0) send16(peer_addr(smem_addr(&s.rcp[par]), b), v, peer_addr(rbar, b));
                 }
             }
             __syncwarp();
             if (jj > 0 && busy) rest(jj - 1);
-            plast = p;
-            if (ok && b == 0 && tid == 0) ipiv[col] = p;
             if (G > 1) {
                 if (ok && !wait_phase(rbar, phase, err)) { ok = false; dev_error(err, M25_DEV_TIMEOUT); }
             } else {
                 __syncthreads();
             }
             if (!ok) *(volatile int *)&s.fail[par ^ 1] = 1;  // (read after the next column's or the group's barrier)
+            const int p = (int)win.p.x;
+            plast = p;
+            if (ok && b == 0 && tid == 0) ipiv[col] = p;
             C rc;
             {
-                const uint4 w = win.rc;
+                const uint4 w = s.rcp[par];
                 memcpy(&rc, &w, sizeof(C));
             }
             const C u0 = win.row[0], u1 = win.row[1];
@@ -353,12 +387,18 @@ __global__ void __launch_bounds__(T, 1) k_panel_cluster(R *A, long lda, int n, i
                 if (b == 0 && lane == 0 && u0.x == 0 && u0.y == 0 && ok) dev_error(err, M25_DEV_ZEROPIV);
             }
         }
+        if (wid == nw - 1 && !dead) {
+            plan(gw - 1);
+            s.pos[lane] = pos;
+            s.src[lane] = src;
+        }
         __syncthreads();
         dead = dead || *(volatile int *)&s.fail[(g0 + gw) & 1];
         if (G > 1 && g0 > 0) cluster_wait();               // the previous group's updates, by all CTAs
         if (!dead) {
-            plan(gw - 1);
             rest(gw - 1);
+            pos = s.pos[lane];
+            src = s.src[lane];
             for (int jj = gw; jj < GRP; ++jj)               // (a short last group: the rotation completed)
 #pragma unroll
                 for (int r = 0; r < RPT; ++r) {
@@ -510,7 +550,7 @@ template <typename R, int GRP, int RPT, int T> int cluster_max()
 // The largest cluster the panel kernel can have on the current device (0: none).
 int m25_panel_cluster_max(int single)
 {
-    return single ? std::min(cluster_max<float, 16, 2, 512>(), cluster_max<float, 8, 4, 512>()) : cluster_max<double, 8, 2, 512>();
+    return single ? std::min(cluster_max<float, 16, 1, 512>(), cluster_max<float, 8, 4, 512>()) : cluster_max<double, 8, 2, 512>();
 }
 
 // Rows the cluster panel takes with cl CTAs of 512 threads: 4 (complex64) or 2 (complex128) rows a thread.
@@ -521,9 +561,9 @@ int m25_panel_cluster_rows(int single, int cl) { return cl * 512 * (single ? 4 :
 // CTAs: one for every 128 rows, up to the cluster's limit (with 64 or 256 rows a CTA the LU of n = 1,000 takes 2-3%
 // longer in complex64, 1-6% in complex128). Per CTA: one row a thread and 16 columns a group as long as the registers
 // allow (groups of 8 at 256 rows: 2-6% longer LUs, twice the group ends), then fewer columns a group and more rows a
-// thread. Whole LUs, complex64 / complex128 with this choice: n = 1,000 2.82 / 3.18 ms, 4,977 16.7 / 22.1 ms; with two
-// rows a thread of 128 for 256 rows 2.83 / 3.31 and 17.5 / 23.2 ms; above 512 rows, complex64, 16 columns and two rows a
-// thread of 512 (spilling) 43.7 against 43.1 ms at n = 9,601.
+// thread. Whole LUs, complex64 / complex128, when the choice was made (both sides are shorter now): n = 1,000 2.82 /
+// 3.18 ms, 4,977 16.7 / 22.1 ms; with two rows a thread of 128 for 256 rows 2.83 / 3.31 and 17.5 / 23.2 ms; above 512
+// rows, complex64, 16 columns and two rows a thread of 512 (spilling) 43.7 against 43.1 ms at n = 9,601.
 int m25_panel_cluster(void *A, long lda, int n, int k0, int jb, int *ipiv, int single, int cl, int *err, cudaStream_t s)
 {
     const int rows = n - k0;

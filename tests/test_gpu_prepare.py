@@ -104,3 +104,30 @@ def test_contour(board, f):
     assert np.abs(got[0] - kr).max() <= 8 * 2.0 ** -53 * K
     assert np.abs(got[1] - dk).max() <= 16 * 2.0 ** -53 * K
     assert np.array_equal(got[0].imag == 0, kr.imag == 0)
+
+
+@pytest.mark.parametrize('nr', [1, 3, 148, 149, 260])
+@pytest.mark.parametrize('ns,npts', [(1, 5), (4, 1025), (5, 300), (16, 700)])
+def test_hankel(ns, npts, nr):
+    """The sums split over four blocks a radius (up to 148 radii) and one, 4, 8 and 16 spectra a pass, complex and real;
+    fewer points than threads too."""
+    from scipy.special import j0, jv
+    from mom25d_b200 import _lib, core
+    from mom25d_b200._lib import P, check, lib
+    rng = np.random.default_rng(nr + npts)
+    c = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)
+    kr = np.linspace(1.0, 900.0, npts) * (1 + 0.02j)
+    kr[npts // 2:] = kr[npts // 2:].real                                   # a contour's tail lies on the real axis
+    dk, W, rho = c(npts), c(ns, npts), np.linspace(1e-4, 0.07, nr)
+    d_kr, d_dk, d_W, d_rho = (_lib.dev(v) for v in (kr, dk, W, rho))
+    out = torch.empty((ns, nr), dtype=torch.complex128, device='cuda')
+    check(lib().m25_hankel(P(d_kr), P(d_dk), npts, P(d_W), ns, P(d_rho), nr, P(out), _lib.stream_ptr()), 'm25_hankel')
+    _lib.sync_check()
+    z = rho[:, None] * kr
+    want = W @ (jv(0, z) * kr * dk).T / (2 * np.pi)
+    # |J0| <= e^|Im z|: each term to 1e-13 of that (J0's accuracy on both sides), and npts additions
+    size = np.abs(W) @ (np.exp(np.abs(z.imag)) * np.abs(kr * dk)).T / (2 * np.pi)
+    assert (np.abs(out.cpu().numpy() - want) <= (2e-13 + npts * 2.0 ** -52) * size).all()
+    got = core.hankel_real(rho, kr.real.copy(), W)
+    want, size = W @ j0(rho[:, None] * kr.real).T, np.abs(W).sum(1)[:, None]
+    assert (np.abs(got - want) <= (2e-13 + npts * 2.0 ** -52) * size).all()
