@@ -1870,7 +1870,8 @@ int lu_streams(LuStreams *out)
 
 // ---- the LU's tile parameters by matrix size (set by the autotuner, mom25d_b200.tune) --------------------------------
 // Two tables, complex64 and complex128, of entries (n, outer panel width, panel blocks); a factorisation of size n
-// takes the entry nearest to n in log n. Without entries: NB2 and min(SMs, 32).
+// takes the panel blocks of the entry nearest to n in log n, and at each outer block the width of the entry nearest to
+// the size of what is left to factor. Without entries: NB2 and min(SMs, 32).
 namespace {
 struct LuTuning { int n, nb2, blocks; };
 LuTuning g_tuning[2][32];
@@ -1896,8 +1897,7 @@ extern "C" int m25_set_lu_tuning(int single, const int *h_n, const int *h_nb2, c
     return M25_OK;
 }
 
-// The parameters a factorisation of size n (complex64 when single) uses: the table's entry nearest in log n, else
-// the defaults; M25_NB2 and M25_PANEL_BLOCKS in the environment override both.
+// The parameters at size n (complex64 when single): the table's entry nearest in log n, else the defaults; M25_NB2 and M25_PANEL_BLOCKS in the environment override both.
 extern "C" int m25_get_lu_tuning(int n, int single, int *nb2, int *blocks)
 {
     int G = sm_count();
@@ -1986,8 +1986,20 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
     // Blocks of the panel: few enough that the cooperative launch finds its SMs quickly while the other stream's
     // update holds the rest (the exchange costs about the same from 37 to 148 blocks), but at least as many as
     // the panel's rows need to fit in shared memory (M25_PANEL_BLOCKS: tuning)
-    int gmax = 32, nb2 = NB2;                                        // outer panel width and panel blocks: the
-    m25_get_lu_tuning(n, sizeof(R) == 4, &nb2, &gmax);               // autotuner's table, else the defaults
+    int gmax = 32;                                                   // panel blocks: the autotuner's table, else the
+    m25_get_lu_tuning(n, sizeof(R) == 4, nullptr, &gmax);            // default
+    // Columns of the outer block at K0: the table's width for a matrix of the size that is left there. A wide block has
+    // fewer and deeper updates of the far columns; a narrow one keeps the critical path short, which decides where those
+    // updates are done before the panels are (the committed table's lines: 64 columns below 2,828 left, then 256 in
+    // complex64, 128 up to 5,477 and 256 in complex128). Measured, 256 columns throughout (complex128: 128 up to 7,000)
+    // against this: complex64 n = 1,000 2.26 / 2.03 ms, 2,921 6.82 / 6.16, 4,977 13.06 / 12.43, 9,601 35.3 / 34.9;
+    // complex128 1,000 2.78 / 2.58, 2,921 8.87 / 8.17, 5,000 21.1 / 20.6, 7,000 44.4 / 43.3.
+    auto width = [&](int K0) -> int {
+        if (K0 >= n) return 0;
+        int w = NB2;
+        m25_get_lu_tuning(n - K0, sizeof(R) == 4, &w, nullptr);
+        return std::min(w, n - K0);
+    };
     const int rows_cap = (int)((size_t)smem_cap / (sizeof(cpx<R>) * NB));   // a block's rows in shared memory
     const int gcap = std::min(G, PANEL_THREADS);                     // a thread of each block reads a block's record
     M25_CHECK(cudaFuncSetAttribute(k_gemm_update<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<R>()));
@@ -2074,9 +2086,10 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
     // L (rows >= KE of columns [K0, KE)), which nothing writes until block k + 1's left interchanges, issued on Lo
     // after this update. Lo's work for a block follows its work for the previous block (stream order).
     bool next_pending = false;
-    for (int K0 = 0; K0 < n; K0 += nb2) {
-        const int JB = std::min(nb2, n - K0), KE = K0 + JB;
-        const int KE2 = std::min(n, KE + nb2), KE3 = std::min(n, KE2 + nb2);
+    for (int K0 = 0, JB; K0 < n; K0 += JB) {
+        JB = width(K0);
+        const int KE = K0 + JB, KE2 = KE + width(KE), KE3 = KE2 + width(KE2);
+        const bool tc = JB > NB;         // (a block of one panel: FP32, as between the panels of a wider one, see below)
         for (int k0 = K0; k0 < KE; k0 += NB) {
             const int jb = std::min(NB, KE - k0);
             int Gp = std::min(gmax, std::max(1, (n - k0 + 31) / 32));
@@ -2110,7 +2123,7 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
         if (KE < n) {                                                       // H: the next block's columns
             if (next_pending) M25_CHECK(cudaStreamWaitEvent(H, ev_next, 0));
             if ((rc = trsm_outer(K0, JB, KE, KE2, H))) return rc;          // interchanges and U12 in one launch
-            if ((rc = gemm(KE, n - KE, KE, KE2 - KE, K0, JB, true, H))) return rc;
+            if ((rc = gemm(KE, n - KE, KE, KE2 - KE, K0, JB, tc, H))) return rc;
         }
         M25_CHECK(cudaStreamWaitEvent(Lo, ev_panel, 0));                    // Lo: the left and the far columns
         if ((rc = laswp(K0, JB, 0, K0, KE2, n, 0, 1, Lo))) return rc;      // (one launch for both)
@@ -2121,10 +2134,10 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
                 if ((rc = trsm(k0, jb, KE2, n, Lo))) return rc;
                 if ((rc = gemm(k0 + jb, KE - k0 - jb, KE2, n - KE2, k0, jb, true, Lo))) return rc;
             }
-            if ((rc = gemm(KE, n - KE, KE2, KE3 - KE2, K0, JB, true, Lo))) return rc;   // block k + 2's columns
+            if ((rc = gemm(KE, n - KE, KE2, KE3 - KE2, K0, JB, tc, Lo))) return rc;   // block k + 2's columns
             M25_CHECK(cudaEventRecord(ev_next, Lo));
             next_pending = true;
-            if ((rc = gemm(KE, n - KE, KE3, n - KE3, K0, JB, true, Lo))) return rc;    // the rest
+            if ((rc = gemm(KE, n - KE, KE3, n - KE3, K0, JB, tc, Lo))) return rc;    // the rest
         }
     }
     M25_CHECK(cudaEventRecord(ev_lo, Lo));                           // the last left interchanges, then the end

@@ -12,13 +12,14 @@ dominant diagonal (pivots away from it as well).
 
 The autotuner times the LU at each size over its host-side parameters and keeps the fastest: for the complex64
 LU with tensor-core updates (the mixed path's factorisation) the number of CTAs of the cooperative panel kernel
-(16 to 64), its outer panel width kept at 256 columns - a narrower one leaves more of the factor's updates to
-3xTF32 instead of FP32 and costs the factor its use as a preconditioner at the low-frequency end (measured on the
-routed board: with 128, the fresh factor at 0.67 GHz no longer converged); for the complex128 LU (the drop-in)
-both the outer panel width (128 / 192 / 256) and the panel CTAs. The winners per size go into TUNING_FILE
-({"device", "sms", "complex64": [{"n", "nb2", "blocks", "ms"}], "complex128": [...]}), which the library reads at
-load (_lib.apply_tuning -> m25_set_lu_tuning): a factorisation takes the entry nearest its size. The tensor-core
-kernel's stage count is a compile-time choice (two stages, two CTAs an SM) and is not searched.
+(16 to 64), with an outer panel width of 256 columns, or of 64 where every update is in FP32 - the widths between
+leave more of the factor's updates to 3xTF32 instead of FP32 and cost the factor its use as a preconditioner at the
+low-frequency end (measured on the routed board: with 128, the fresh factor at 0.67 GHz no longer converged); for the
+complex128 LU (the drop-in) both the outer panel width (64 / 128 / 192 / 256) and the panel CTAs. The winners per size
+go into TUNING_FILE ({"device", "sms", "complex64": [{"n", "nb2", "blocks", "ms"}], "complex128": [...]}), which the
+library reads at load (_lib.apply_tuning -> m25_set_lu_tuning): a factorisation takes the panel CTAs of the entry
+nearest its size, and for each outer panel the width of the entry nearest the size that is left to factor. The
+tensor-core kernel's stage count is a compile-time choice (two stages, two CTAs an SM) and is not searched.
 """
 import os
 import argparse
@@ -43,8 +44,8 @@ def random_matrix(n, dtype, seed=0):
 
 
 TUNING_FILE = os.path.join(os.path.dirname(os.path.abspath(__file__)), 'tuning_b200.json')
-GRIDS = {True: [(256, bl) for bl in (16, 24, 32, 48, 64)],
-         False: [(b2, bl) for b2 in (128, 192, 256) for bl in (16, 32, 48)]}
+GRIDS = {True: [(256, bl) for bl in (16, 24, 32, 48, 64)] + [(64, 32)],
+         False: [(b2, bl) for b2 in (64, 128, 192, 256) for bl in (16, 32, 48)]}
 
 
 def set_table(entries, single=True):
@@ -60,7 +61,7 @@ def autotune(sizes, single=True, reps=2, log=print):
     for n in sizes:
         grid = GRIDS[single]
         if n > 30000:                                     # (the largest size: a coarser grid, each LU is seconds)
-            grid = [g for g in grid if g[1] in (32, 48)][:4]
+            grid = [g for g in grid if g[0] > 64 and g[1] in (32, 48)][:4]
         times = {}
         for b2, bl in grid:
             set_table([(1, b2, bl)], single)
