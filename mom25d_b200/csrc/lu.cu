@@ -14,7 +14,9 @@
 //                  (umma.cu) for complex64 with tf32 on.
 #include <type_traits>
 #include <algorithm>
+#include <memory>
 #include <mutex>
+#include <new>
 
 #include "common.cuh"
 
@@ -764,9 +766,9 @@ template <typename R> constexpr size_t t64_smem()
 // takes a row below the block and subtracts the block's multiples from it for all the CTA's columns (L read from
 // the factor, coalesced across the threads, a batch ahead of its use, as the next diagonal block is). Each entry takes
 // its terms x -= L(k, i) x_i in ascending i, as a forward substitution does; FP32 (FP64) on the CUDA cores throughout.
-// Latency-bound: few columns, a chain of JB rows. In the complex64 LU of n = 4,977, 15 us on average over its 58 panels
-// of 64 (192 columns or fewer; a thread a column, k_trsm64, took 30) and 19 outer panels of 256 (66 with every entry of
-// L read where it is used).
+// Latency-bound: few columns, a chain of JB rows. In a complex64 LU of n = 4,977 with outer panels of 256 throughout, 15
+// us on average over its 58 panels of 64 (192 columns or fewer; a thread a column, k_trsm64, took 30) and 19 outer panels
+// of 256 (66 with every entry of L read where it is used).
 #define TO_COLS 8
 #define TO_THREADS 256
 static_assert(TO_COLS * 32 == TO_THREADS, "a warp a column");
@@ -959,13 +961,14 @@ __global__ void __launch_bounds__(256) k_gemm_update(R *Cm, const R *Am, const R
     }
 }
 
-// The same for K <= 64 in complex64 (the updates inside an outer panel, at most 192 columns wide): the whole depth of
+// The same for K <= 64 in complex64 (the FP32 updates by one panel: of the columns the next panels need, and in outer
+// blocks of one panel of everything to the right): the whole depth of
 // both operands is copied into shared memory at once (cp.async, 8 bytes: a factor's columns need not be 16-byte aligned)
 // in four groups of 16, the products of a group start as it lands, and C is read ahead of them. BM rows x 64 columns a
 // block of 256 threads, each BM / 16 x 4 outputs; BM = 64 where 128 rows a block would leave SMs idle. Each entry takes
 // its terms in k order, as k_gemm_update adds them. What bounds it is one SM's FP32 rate (8 us for 128 x 64 x 64).
-// n = 4,977: 24 us an update by k_gemm_update (slices of 8, rows of C 16 bytes at a time), 13 with BM = 64 (M below
-// about 4,700 rows), 19 with BM = 128 (above).
+// n = 4,977, up to 192 columns: 24 us an update by k_gemm_update (slices of 8, rows of C 16 bytes at a time), 13 with
+// BM = 64 (M below about 4,700 rows), 19 with BM = 128 (above).
 __device__ __forceinline__ void cp_async8_zfill(void *smem, const void *gmem, bool valid)
 {
     unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
@@ -1841,13 +1844,14 @@ extern "C" size_t m25_getrf_workspace(int n, int single)
     return b;
 }
 
-// The LU's two internal streams on the current device: a high-priority one for the panels and everything on the
-// critical path, a low-priority one for the trailing update of the previous outer block, so that the next block's
-// panels run while that update does (look-ahead); and the events between them. One set per host thread and device,
+// The LU's internal streams on the current device: a high-priority one for the panels and everything on the critical
+// path, a low-priority one for the trailing update of the previous outer block, so that the next block's panels run
+// while that update does (look-ahead), and one between them for the columns that the panels after the next one need;
+// and the events between them. One set per host thread and device,
 // created on the thread's first factorisation there (calls from different threads, e.g. concurrent requests on
 // their own streams, do not share them; calls from one thread are ordered by it).
 namespace {
-struct LuStreams { cudaStream_t hi = nullptr, lo = nullptr; cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr}; };
+struct LuStreams { cudaStream_t hi = nullptr, mid = nullptr, lo = nullptr; cudaEvent_t ev[7] = {}; };
 thread_local LuStreams g_lu[64];
 
 int lu_streams(LuStreams *out)
@@ -1860,6 +1864,7 @@ int lu_streams(LuStreams *out)
         int least = 0, greatest = 0;
         M25_CHECK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
         M25_CHECK(cudaStreamCreateWithPriority(&L.hi, cudaStreamNonBlocking, greatest));
+        M25_CHECK(cudaStreamCreateWithPriority(&L.mid, cudaStreamNonBlocking, (least + greatest) / 2));
         M25_CHECK(cudaStreamCreateWithPriority(&L.lo, cudaStreamNonBlocking, least));
         for (auto &e : L.ev) M25_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
@@ -1955,8 +1960,10 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
     int rc = lu_streams(&st);
     if (rc) return rc;
     const char *la = getenv("M25_LOOKAHEAD");                       // 0: one stream (the same results, in order)
-    const cudaStream_t H = st.hi, Lo = (la && atoi(la) == 0) ? st.hi : st.lo;
-    cudaEvent_t ev_start = st.ev[0], ev_panel = st.ev[1], ev_next = st.ev[2], ev_lo = st.ev[3], ev_end = st.ev[4];
+    const bool one = la && atoi(la) == 0;
+    const cudaStream_t H = st.hi, Mid = one ? st.hi : st.mid, Lo = one ? st.hi : st.lo;
+    cudaEvent_t ev_start = st.ev[0], ev_panel = st.ev[1], ev_next = st.ev[2], ev_lo = st.ev[3], ev_end = st.ev[4],
+                ev_col = st.ev[5], ev_mid = st.ev[6];
     M25_CHECK(cudaEventRecord(ev_start, s));                        // the caller's work first
     M25_CHECK(cudaStreamWaitEvent(H, ev_start, 0));
     M25_CHECK(cudaStreamWaitEvent(Lo, ev_start, 0));
@@ -1988,18 +1995,20 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
     // the panel's rows need to fit in shared memory (M25_PANEL_BLOCKS: tuning)
     int gmax = 32;                                                   // panel blocks: the autotuner's table, else the
     m25_get_lu_tuning(n, sizeof(R) == 4, nullptr, &gmax);            // default
-    // Columns of the outer block at K0: the table's width for a matrix of the size that is left there. A wide block has
-    // fewer and deeper updates of the far columns; a narrow one keeps the critical path short, which decides where those
-    // updates are done before the panels are (the committed table's lines: 64 columns below 2,828 left, then 256 in
-    // complex64, 128 up to 5,477 and 256 in complex128). Measured, 256 columns throughout (complex128: 128 up to 7,000)
-    // against this: complex64 n = 1,000 2.26 / 2.03 ms, 2,921 6.82 / 6.16, 4,977 13.06 / 12.43, 9,601 35.3 / 34.9;
-    // complex128 1,000 2.78 / 2.58, 2,921 8.87 / 8.17, 5,000 21.1 / 20.6, 7,000 44.4 / 43.3.
-    auto width = [&](int K0) -> int {
-        if (K0 >= n) return 0;
-        int w = NB2;
-        m25_get_lu_tuning(n - K0, sizeof(R) == 4, &w, nullptr);
-        return std::min(w, n - K0);
-    };
+    // Columns of an outer block: the table's width for a matrix of the size that is left there. A wide block has fewer
+    // and deeper updates of the far columns; a narrow one keeps the critical path short, which decides where those
+    // updates are done before the panels are (the committed table's lines: 64 columns below 2,828 left, 128 below 5,000
+    // in complex64 and 5,477 in complex128, 256 above). Measured, one width throughout (complex64 256; complex128 128,
+    // at 9,601 256) against this: complex64 n = 1,000 2.26 / 2.03 ms, 2,921 6.82 / 6.15, 4,977 13.1 / 12.1, 7,000
+    // 20.9 / 19.3; complex128 1,000 2.78 / 2.58, 2,921 8.87 / 8.17, 5,000 21.1 / 20.6, 7,000 44.4 / 43.3.
+    const std::unique_ptr<int[]> start(new (std::nothrow) int[n / NB + 1]);    // first columns, read once (another
+    M25_REQUIRE(start, "m25_getrf: out of host memory");                       // thread may set the table)
+    int nblk = 0;
+    for (int k = 0, w = NB2; k < n; k += w) {                        // (w >= NB)
+        start[nblk++] = k;
+        m25_get_lu_tuning(n - k, sizeof(R) == 4, &w, nullptr);
+    }
+    auto at = [&](int i) { return i < nblk ? start[i] : n; };
     const int rows_cap = (int)((size_t)smem_cap / (sizeof(cpx<R>) * NB));   // a block's rows in shared memory
     const int gcap = std::min(G, PANEL_THREADS);                     // a thread of each block reads a block's record
     M25_CHECK(cudaFuncSetAttribute(k_gemm_update<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<R>()));
@@ -2082,14 +2091,22 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
     //   Lo (low priority): as soon as block k's panels are done (ev_panel), block k's interchanges on the columns
     //     left of it and on [KE2, n), U12 of [KE2, n), then the update of [KE2, n): first the columns of block
     //     k + 2 ([KE2, KE3): ev_next, which H waits for at block k + 1), then the rest.
+    // In complex64 with at most WIN_ROWS rows left the critical path is one panel's columns at a time instead: after
+    // each panel H updates the next panel's columns alone (in this block or the next), and Mid the columns after those
+    // up to KE2, by that panel (ev_col), while H factors the next one; H waits for that (ev_mid) before it updates a
+    // column Mid has worked on. So the next block's columns are done when block k's last panel is, in FP32, and H has
+    // no outer step. (n = 4,977 12.43 -> 12.11 ms, 7,000 20.2 -> 19.3; with more rows left the far update has no
+    // SMs to spare: n = 12,000 with this for every size 50.3 -> 51.4, 18,788 151.9 -> 155.7. In complex128, whose far
+    // update takes most of the time from 2,700 rows on, 4,000 went from 13.03 to 13.29.)
     // Regions: H works on columns >= KE only; Lo on columns < K0 (interchanges) and >= KE2; both read block k's
     // L (rows >= KE of columns [K0, KE)), which nothing writes until block k + 1's left interchanges, issued on Lo
     // after this update. Lo's work for a block follows its work for the previous block (stream order).
-    bool next_pending = false;
-    for (int K0 = 0, JB; K0 < n; K0 += JB) {
-        JB = width(K0);
-        const int KE = K0 + JB, KE2 = KE + width(KE), KE3 = KE2 + width(KE2);
-        const bool tc = JB > NB;         // (a block of one panel: FP32, as between the panels of a wider one, see below)
+    constexpr int WIN_ROWS = sizeof(R) == 4 ? 8000 : 0;
+    bool next_pending = false, mid_pending = false;
+    for (int blk = 0; blk < nblk; ++blk) {
+        const int K0 = at(blk), KE = at(blk + 1), KE2 = at(blk + 2), KE3 = at(blk + 3), JB = KE - K0;
+        const bool win = n - K0 <= WIN_ROWS;
+        const bool tc = JB > NB;             // (a block of one panel: FP32, as between a wider one's panels, see below)
         for (int k0 = K0; k0 < KE; k0 += NB) {
             const int jb = std::min(NB, KE - k0);
             int Gp = std::min(gmax, std::max(1, (n - k0 + 31) / 32));
@@ -2109,6 +2126,23 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
                 M25_CHECK(cudaLaunchCooperativeKernel((void *)k_panel<R>, dim3(Gp), dim3(PANEL_THREADS), args, 0, H));
                 m25_note_launch();
             }
+            if (win) {
+                const int c0 = k0 + jb, c1 = std::min(n, c0 + NB);         // the next panel's columns
+                M25_CHECK(cudaEventRecord(ev_col, H));
+                if (c0 == KE && next_pending) M25_CHECK(cudaStreamWaitEvent(H, ev_next, 0));
+                if (mid_pending) M25_CHECK(cudaStreamWaitEvent(H, ev_mid, 0));
+                if ((rc = trsm_outer(k0, jb, c0, c1, H))) return rc;
+                if ((rc = gemm(c0, n - c0, c0, c1 - c0, k0, jb, false, H))) return rc;
+                if (c1 < KE2) {
+                    if (k0 == K0 && next_pending) M25_CHECK(cudaStreamWaitEvent(Mid, ev_next, 0));
+                    M25_CHECK(cudaStreamWaitEvent(Mid, ev_col, 0));
+                    if ((rc = trsm_outer(k0, jb, c1, KE2, Mid))) return rc;
+                    if ((rc = gemm(c0, n - c0, c1, KE2 - c1, k0, jb, false, Mid))) return rc;
+                    M25_CHECK(cudaEventRecord(ev_mid, Mid));
+                    mid_pending = true;
+                }
+                continue;
+            }
             if ((rc = trsm_outer(k0, jb, k0 + jb, KE, H))) return rc;      // the rest of the outer panel
             // in FP32 on the CUDA cores, not 3xTF32: the columns of L pass through every update of their outer
             // panel, and the tensor-core error there (about 2^-22 a product against 2^-24) costs the factor its
@@ -2116,16 +2150,22 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
             // board no longer converged; the FP32 inner update costs 5 ms of 236 at N = 18,788)
             if ((rc = gemm(k0 + jb, n - k0 - jb, k0 + jb, KE - k0 - jb, k0, jb, false, H))) return rc;
         }
-        // each earlier panel's columns of the outer panel: the interchanges of the panels after it (one launch)
+        // each earlier panel's columns of the outer panel: the interchanges of the panels after it (one launch; on Lo
+        // where H needs a panel's columns only right after it)
         const int npan = (JB + NB - 1) / NB;
-        if (npan > 1 && (rc = laswp(K0 + NB, JB - NB, K0, K0 + NB, 0, 0, NB, npan - 1, H))) return rc;
+        auto swap_block = [&](cudaStream_t cs) -> int {
+            return npan > 1 ? laswp(K0 + NB, JB - NB, K0, K0 + NB, 0, 0, NB, npan - 1, cs) : M25_OK;
+        };
+        if (!win && (rc = swap_block(H))) return rc;
         M25_CHECK(cudaEventRecord(ev_panel, H));                          // block k's L and pivots are final
-        if (KE < n) {                                                       // H: the next block's columns
+        if (KE < n && !win) {                                               // H: the next block's columns
             if (next_pending) M25_CHECK(cudaStreamWaitEvent(H, ev_next, 0));
             if ((rc = trsm_outer(K0, JB, KE, KE2, H))) return rc;          // interchanges and U12 in one launch
             if ((rc = gemm(KE, n - KE, KE, KE2 - KE, K0, JB, tc, H))) return rc;
         }
         M25_CHECK(cudaStreamWaitEvent(Lo, ev_panel, 0));                    // Lo: the left and the far columns
+        if (mid_pending) M25_CHECK(cudaStreamWaitEvent(Lo, ev_mid, 0));     // (Mid reads L before its interchanges)
+        if (win && (rc = swap_block(Lo))) return rc;
         if ((rc = laswp(K0, JB, 0, K0, KE2, n, 0, 1, Lo))) return rc;      // (one launch for both)
         next_pending = false;
         if (KE2 < n) {

@@ -14,12 +14,15 @@ The autotuner times the LU at each size over its host-side parameters and keeps 
 LU with tensor-core updates (the mixed path's factorisation) the number of CTAs of the cooperative panel kernel
 (16 to 64), with an outer panel width of 256 columns, or of 64 where every update is in FP32 - the widths between
 leave more of the factor's updates to 3xTF32 instead of FP32 and cost the factor its use as a preconditioner at the
-low-frequency end (measured on the routed board: with 128, the fresh factor at 0.67 GHz no longer converged); for the
-complex128 LU (the drop-in) both the outer panel width (64 / 128 / 192 / 256) and the panel CTAs. The winners per size
-go into TUNING_FILE ({"device", "sms", "complex64": [{"n", "nb2", "blocks", "ms"}], "complex128": [...]}), which the
-library reads at load (_lib.apply_tuning -> m25_set_lu_tuning): a factorisation takes the panel CTAs of the entry
-nearest its size, and for each outer panel the width of the entry nearest the size that is left to factor. The
-tensor-core kernel's stage count is a compile-time choice (two stages, two CTAs an SM) and is not searched.
+low-frequency end (measured on the routed board: with 128, the fresh factor at 0.67 GHz no longer converged). With at
+most 8,000 rows left the next block's columns too are updated in FP32, which makes up for a narrower block: the
+committed file's 128 columns at 4,000 are of that kind (n = 4,977: residual of the factor 0.9e-4 against 1.7e-4 with
+256 and the next block's columns in 3xTF32) and are entered by hand. For the complex128 LU (the drop-in) both the outer
+panel width (64 / 128 / 192 / 256) and the panel CTAs are searched. The winners per size go into TUNING_FILE
+({"device", "sms", "complex64": [{"n", "nb2", "blocks", "ms"}], "complex128": [...]}), which the library reads at
+load (_lib.apply_tuning -> m25_set_lu_tuning): a factorisation takes the panel CTAs of the entry nearest its size, and
+for each outer panel the width of the entry nearest the size that is left to factor. The tensor-core kernel's stage
+count is a compile-time choice (two stages, two CTAs an SM) and is not searched.
 """
 import os
 import argparse

@@ -9,8 +9,8 @@ pytestmark = pytest.mark.gpu
 
 torch = pytest.importorskip('torch')
 
-TABLES = {'falling': [(100, 64), (250, 128), (500, 192), (1000, 256)], 'mixed': [(150, 128), (300, 64), (600, 256), (900, 64)],
-          'committed': None}
+TABLES = {'falling': [(100, 64), (250, 128), (500, 192), (1000, 256)],
+          'mixed': [(150, 128), (300, 64), (600, 256), (900, 64)], 'committed': None}
 
 
 @pytest.mark.parametrize('n', [64, 65, 129, 300, 449, 700, 1100])
