@@ -50,6 +50,20 @@ template <typename R> __host__ __device__ __forceinline__ void cfms(cpx<R> &a, c
 typedef cpx<double> zd;
 typedef cpx<float> zf;
 
+// N complex entries that are moved as 16-byte pieces. A cpx is aligned to its element only (4 or 8 bytes), and so is an
+// array of them: wherever one is kept in memory (shared, or a thread's own when it does not fit its registers) a
+// 16-byte access needs the alignment from the type.
+template <typename R, int N> struct __align__(16) cpx_row {
+    cpx<R> c[N];
+    static constexpr int PIECES = N * (int)sizeof(cpx<R>) / 16;
+    static_assert(N * sizeof(cpx<R>) % 16 == 0, "whole pieces, and rows of an array on 16-byte boundaries");
+    __device__ __forceinline__ cpx<R> &operator[](int i) { return c[i]; }
+    __device__ __forceinline__ const cpx<R> &operator[](int i) const { return c[i]; }
+    __device__ __forceinline__ uint4 &piece(int q) { return reinterpret_cast<uint4 *>(c)[q]; }
+    __device__ __forceinline__ const uint4 &piece(int q) const { return reinterpret_cast<const uint4 *>(c)[q]; }
+};
+static_assert(alignof(cpx_row<float, 8>) == 16 && alignof(cpx_row<double, 8>) == 16, "16-byte pieces");
+
 template <typename R> __device__ __forceinline__ cpx<R> ldc(const R *p, size_t i)
 {
     typedef typename vec2_of<R>::type V;

@@ -783,8 +783,9 @@ __global__ void __launch_bounds__(TO_THREADS) k_trsm_outer(R *A, long lda, int n
     constexpr int CH = sizeof(R) == 4 ? 16 : 8;            // terms of a row below in flight
     extern __shared__ __align__(16) unsigned char to_raw[];
     __shared__ SwapPlan P;
-    C *X = reinterpret_cast<C *>(to_raw);                 // X[r * TO_COLS + j]: row K0 + r of the CTA's column j
-    C *Lb = X + (size_t)NB2 * TO_COLS;                     // Lb[i * (NB + 1) + k] = L11(kb + k, kb + i)
+    typedef cpx_row<R, TO_COLS> Row;
+    Row *X = reinterpret_cast<Row *>(to_raw);             // X[r][j]: row K0 + r of the CTA's column j
+    C *Lb = reinterpret_cast<C *>(X + NB2);                // Lb[i * (NB + 1) + k] = L11(kb + k, kb + i)
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const long cw = c0 + (long)blockIdx.x * TO_COLS + w;    // this warp's column
     C lq[LQ];                                              // the next diagonal block on its way to Lb
@@ -807,10 +808,10 @@ __global__ void __launch_bounds__(TO_THREADS) k_trsm_outer(R *A, long lda, int n
     swap_plan(ipiv, K0, JB, n, P, err);
     {
         long cs[1] = {cw < c1 ? cw : -1};
-        if (JB <= NB) apply_plan<R, 2 * NB / 32, 1>(A, lda, cs, P, lane, X + w, JB, 0, TO_COLS);
-        else apply_plan<R, 2 * PLAN_MAX / 32, 1>(A, lda, cs, P, lane, X + w, JB, 0, TO_COLS);
+        if (JB <= NB) apply_plan<R, 2 * NB / 32, 1>(A, lda, cs, P, lane, X[0].c + w, JB, 0, TO_COLS);
+        else apply_plan<R, 2 * PLAN_MAX / 32, 1>(A, lda, cs, P, lane, X[0].c + w, JB, 0, TO_COLS);
         if (cw >= c1)
-            for (int r = lane; r < JB; r += 32) X[r * TO_COLS + w] = mk<R>(0, 0);
+            for (int r = lane; r < JB; r += 32) X[r][w] = mk<R>(0, 0);
     }
     store();
     __syncthreads();
@@ -819,8 +820,8 @@ __global__ void __launch_bounds__(TO_THREADS) k_trsm_outer(R *A, long lda, int n
         const bool more = kb + jb < JB;                    // (then jb == NB)
         if (more) fetch(kb + jb);
         {                                                  // the diagonal block, warp w's column
-            C x0 = lane < jb ? X[(kb + lane) * TO_COLS + w] : mk<R>(0, 0);
-            C x1 = lane + 32 < jb ? X[(kb + lane + 32) * TO_COLS + w] : mk<R>(0, 0);
+            C x0 = lane < jb ? X[kb + lane][w] : mk<R>(0, 0);
+            C x1 = lane + 32 < jb ? X[kb + lane + 32][w] : mk<R>(0, 0);
 #pragma unroll 4
             for (int i = 0; i < min(32, jb - 1); ++i) {
                 C xi;
@@ -836,18 +837,17 @@ __global__ void __launch_bounds__(TO_THREADS) k_trsm_outer(R *A, long lda, int n
                 xi.y = __shfl_sync(0xffffffffu, x1.y, i - 32);
                 if (lane + 32 > i) cfms<R>(x1, Lb[i * (NB + 1) + lane + 32], xi);
             }
-            if (lane < jb) X[(kb + lane) * TO_COLS + w] = x0;
-            if (lane + 32 < jb) X[(kb + lane + 32) * TO_COLS + w] = x1;
+            if (lane < jb) X[kb + lane][w] = x0;
+            if (lane + 32 < jb) X[kb + lane + 32][w] = x1;
         }
         __syncthreads();
         if (!more) break;
         const int r = kb + NB + t;                          // the rows below the block (at most NB2 - NB: one a thread)
         if (r < JB) {
-            C x[TO_COLS], lv[CH];
-            uint4 *xr = reinterpret_cast<uint4 *>(X + r * TO_COLS);
-            constexpr int XQ = TO_COLS * (int)sizeof(C) / 16;
+            Row x;
+            C lv[CH];
 #pragma unroll
-            for (int q = 0; q < XQ; ++q) reinterpret_cast<uint4 *>(x)[q] = xr[q];
+            for (int q = 0; q < Row::PIECES; ++q) x.piece(q) = X[r].piece(q);
             const R *lr = A + 2 * ((size_t)(K0 + kb) * lda + K0 + r);
 #pragma unroll
             for (int q = 0; q < CH; ++q) lv[q] = ldc<R>(lr, (size_t)q * lda);
@@ -857,10 +857,9 @@ __global__ void __launch_bounds__(TO_THREADS) k_trsm_outer(R *A, long lda, int n
                 for (int q = 0; q < CH; ++q) ln[q] = i + CH < NB ? ldc<R>(lr, (size_t)(i + CH + q) * lda) : mk<R>(0, 0);
 #pragma unroll
                 for (int q = 0; q < CH; ++q) {
-                    C xi[TO_COLS];
-                    const uint4 *xp = reinterpret_cast<const uint4 *>(X + (kb + i + q) * TO_COLS);
+                    Row xi;
 #pragma unroll
-                    for (int h = 0; h < XQ; ++h) reinterpret_cast<uint4 *>(xi)[h] = xp[h];
+                    for (int h = 0; h < Row::PIECES; ++h) xi.piece(h) = X[kb + i + q].piece(h);
 #pragma unroll
                     for (int j = 0; j < TO_COLS; ++j) cfms<R>(x[j], lv[q], xi[j]);
                 }
@@ -868,13 +867,13 @@ __global__ void __launch_bounds__(TO_THREADS) k_trsm_outer(R *A, long lda, int n
                 for (int q = 0; q < CH; ++q) lv[q] = ln[q];
             }
 #pragma unroll
-            for (int q = 0; q < XQ; ++q) xr[q] = reinterpret_cast<uint4 *>(x)[q];
+            for (int q = 0; q < Row::PIECES; ++q) X[r].piece(q) = x.piece(q);
         }
         store();                                           // (the diagonal block's reads of Lb ended at the barrier)
         __syncthreads();
     }
     if (cw < c1)
-        for (int r = lane; r < JB; r += 32) stc<R>(A, (size_t)cw * lda + K0 + r, X[r * TO_COLS + w]);
+        for (int r = lane; r < JB; r += 32) stc<R>(A, (size_t)cw * lda + K0 + r, X[r][w]);
 }
 static_assert(NB2 - NB <= TO_THREADS, "a thread a row below the first block");
 

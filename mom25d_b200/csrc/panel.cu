@@ -122,15 +122,16 @@ __device__ __forceinline__ uint4 piece_of(cpx<double> x, int)        // (an entr
 
 template <typename R, int GRP> struct PanelShared {
     typedef cpx<R> C;
-    static constexpr int RB = GRP * (int)sizeof(C) / 16;              // 16-byte pieces of a row's GRP entries
+    typedef cpx_row<R, GRP> Entries;
+    static constexpr int RB = Entries::PIECES;                        // 16-byte pieces of a row's GRP entries
     uint4 head[2][PCL_MAX];                  // each CTA's candidate's entry (NaN: none), by column parity
-    struct __align__(16) Row { C row[GRP]; uint4 p; } win[2];         // the pivot row and its index
+    struct Row { Entries row; uint4 p; } win[2];                      // the pivot row and its index
     uint4 rcp[2];                            // 1 / pivot
     int pos[32], src[32];                    // the group's interchanges (plan), for the other columns
-    C diag[2][GRP];                          // the diagonal row, in the CTA of the pivot row
-    struct __align__(16) Stage { C row[GRP]; C l, next; } stage[2];   // a row on its way out: candidate, diagonal row
+    Entries diag[2];                         // the diagonal row, in the CTA of the pivot row
+    struct Stage { Entries row; C l, next; } stage[2];                // a row on its way out: candidate, diagonal row
     C prow[GRP][GRP];                        // the group's pivot rows (rotated as they were sent)
-    C u[PNB][GRP];                           // the group's rows of U on the columns to the right
+    Entries u[PNB];                          // the group's rows of U on the columns to the right
     uint4 cand[2][16];                       // the warps' candidates, by column parity
     int fail[2];                             // a wait of this CTA gave up in the column before (by column parity)
     unsigned long long bar[4];               // of the candidates, then of the rows, by column parity
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(T, 1) k_panel_cluster(R *A, long lda, int n, i
     const int cs = (n - k0 + G - 1) / G, r0 = k0 + b * cs, nr = max(0, min(n, r0 + cs) - r0);
     const int rend = r0 + nr;
     const uint32_t bar0 = smem_addr(&s.bar[0]);
-    C a[RPT][GRP];
+    typename PS::Entries a[RPT];
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
         const int row = r0 + tid + T * r;
@@ -193,7 +194,7 @@ __global__ void __launch_bounds__(T, 1) k_panel_cluster(R *A, long lda, int n, i
         C l[RPT], next[RPT];
         auto rest = [&](int jj) {
             const int col = gr + jj;
-            const C *urow = s.win[(g0 + jj) & 1].row;
+            const typename PS::Entries &urow = s.win[(g0 + jj) & 1].row;
 #pragma unroll
             for (int c = 2; c < GRP; ++c) {
                 const C u = urow[c];
@@ -215,10 +216,8 @@ __global__ void __launch_bounds__(T, 1) k_panel_cluster(R *A, long lda, int n, i
 #pragma unroll
             for (int r = 0; r < RPT; ++r)
                 if (r0 + tid + T * r == row) {
-                    uint4 *d = reinterpret_cast<uint4 *>(st.row);
-                    const uint4 *ar = reinterpret_cast<const uint4 *>(a[r]);
 #pragma unroll
-                    for (int q = 0; q < RB; ++q) d[q] = ar[q];
+                    for (int q = 0; q < RB; ++q) st.row.piece(q) = a[r].piece(q);
                     st.l = l[r];
                     st.next = next[r];
                 }
@@ -328,13 +327,13 @@ __global__ void __launch_bounds__(T, 1) k_panel_cluster(R *A, long lda, int n, i
                         }
                         if (lane < G) send16(peer_addr(smem_addr(&win.p), lane), pi, peer_addr(rbar, lane));
                     } else {
-                        if (lane < RB) reinterpret_cast<uint4 *>(win.row)[lane] = cp;
+                        if (lane < RB) win.row.piece(lane) = cp;
                         if (lane == 0) win.p = pi;
                     }
                 }
                 if (wid == dw && swap && lane < RB) {
                     if (G > 1) send16(peer_addr(smem_addr(&s.diag[par][0]) + 16 * lane, wq), dp, peer_addr(rbar, wq));
-                    else reinterpret_cast<uint4 *>(s.diag[par])[lane] = dp;
+                    else s.diag[par].piece(lane) = dp;
                 }
                 const int helper = cw != 0 && dw != 0 ? 0 : cw != 1 && dw != 1 ? 1 : 2;
                 if (G > 1 && wid == helper) {
@@ -366,9 +365,9 @@ __global__ void __launch_bounds__(T, 1) k_panel_cluster(R *A, long lda, int n, i
             for (int r = 0; r < RPT; ++r) {
                 const int row = r0 + tid + T * r;
                 if (row == col || row == p) {
-                    const uint4 *from = reinterpret_cast<const uint4 *>(row == col ? win.row : s.diag[par]);
+                    const typename PS::Entries &from = row == col ? win.row : s.diag[par];
 #pragma unroll
-                    for (int q = 0; q < RB; ++q) reinterpret_cast<uint4 *>(a[r])[q] = from[q];
+                    for (int q = 0; q < RB; ++q) a[r].piece(q) = from.piece(q);
                 }
                 const C a0 = a[r][0], v = a[r][1], t = a0 * rc;
                 const bool act = row > col;
@@ -466,11 +465,10 @@ __global__ void __launch_bounds__(T, 1) k_panel_cluster(R *A, long lda, int n, i
                 s.u[c][i] = ldc_l2<R>(A, (size_t)(gr + GRP + c) * lda + gr + i);
             }
             __syncthreads();
-            auto upd = [&](C &v, const C (&l)[GRP], int c) {
-                const uint4 *u = reinterpret_cast<const uint4 *>(s.u[c]);
+            auto upd = [&](C &v, const typename PS::Entries &l, int c) {
 #pragma unroll
                 for (int q = 0; q < RB; ++q) {
-                    const uint4 w = u[q];
+                    const uint4 w = s.u[c].piece(q);
                     const C *uc = reinterpret_cast<const C *>(&w);
 #pragma unroll
                     for (int h = 0; h < 16 / (int)sizeof(C); ++h) cfms<R>(v, l[q * (16 / (int)sizeof(C)) + h], uc[h]);
