@@ -29,13 +29,14 @@ GAUSS = {nq: np.polynomial.legendre.leggauss(nq) for nq in (8,)}        # the co
 
 def contour_path(f, st, rho_max, K=None):
     """The pieces of the Sommerfeld integration path (via.py:36-53): lifted into the upper half plane by alpha sin up to
-    t1 = 1.5 k_max in m1 equal pieces, then real to K in pieces of wid2, n2 of them: (t1, alpha, K, wid2, m1, n2)."""
+    t1 = 1.5 k_max in m1 equal pieces, then real to K in pieces of wid2, n2 of them (none where K <= t1: the path ends at
+    t1): (t1, alpha, K, wid2, m1, n2)."""
     k0 = 2 * np.pi * f / C0
     kmax = k0 * np.sqrt(st.max_er())
     K = K or (max(1e5, 30.0 / st.hmin) + 40 * kmax)
     t1, alpha = 1.5 * kmax, min(0.5 * k0, 4.0 / rho_max)
     wid1, wid2 = min(0.3 * k0, 0.8 * alpha), 2 * np.pi / rho_max
-    return t1, alpha, K, wid2, int(np.ceil(t1 / wid1)), int(np.ceil((K - t1) / wid2))
+    return t1, alpha, K, wid2, int(np.ceil(t1 / wid1)), max(0, int(np.ceil((K - t1) / wid2)))
 
 
 def sommerfeld_contour(f, st, rho_max, K=None, nq=8):
@@ -43,7 +44,7 @@ def sommerfeld_contour(f, st, rho_max, K=None, nq=8):
     m25_contour's)."""
     t1, alpha, K, wid2, m1, n2 = contour_path(f, st, rho_max, K)
     xg, wg = GAUSS[nq] if nq in GAUSS else np.polynomial.legendre.leggauss(nq)
-    br = np.concatenate([np.linspace(0, t1, m1 + 1), t1 + wid2 * np.arange(1, n2), [K]])
+    br = np.concatenate([np.linspace(0, t1, m1 + 1), t1 + wid2 * np.arange(1, n2), [K] if n2 else []])
     a, b = br[:-1, None], br[1:, None]
     t = (0.5 * (b - a) * xg[None, :] + 0.5 * (a + b)).ravel()
     wt = (0.5 * (b - a) * wg[None, :]).ravel()
