@@ -664,19 +664,20 @@ class DirectSolver:
             hist.append(res.copy())
             if done.all():
                 return True
+            return ends(j + 1, res)
+
+        def ends(n, r):
+            """Whether the iteration is given up after n steps where the columns' residuals are r then."""
             act = ~done
-            if give_up is not None and j + 1 >= give_up[0] and j + 1 < restart and \
-                    (res[act] > give_up[1] * bn[act]).any():
+            if give_up is not None and give_up[0] <= n < restart and (r[act] > give_up[1] * bn[act]).any():
                 return True
-            if stagnate is not None and j + 1 == stagnate[0] and j + 1 < restart and \
-                    (res[act] > stagnate[1] * hist[1][act]).any():
+            if stagnate is not None and n == stagnate[0] and n < restart and (r[act] > stagnate[1] * hist[1][act]).any():
                 return True
-            if stall is not None and j + 1 >= stall[0] and (res[act] > stall[1] * bn[act]).any():
+            if stall is not None and n >= stall[0] and (r[act] > stall[1] * bn[act]).any():
                 return True
-            if stall is not None and predict and j + 1 >= PREDICT_AFTER:
-                rate = (res[act] / bn[act]) ** (1.0 / (j + 1))
-                if (res[act] * rate ** (restart - j - 1) > 10 * rtol * bn[act]).any():
-                    return True
+            if stall is not None and predict and n >= PREDICT_AFTER:
+                rate = (r[act] / bn[act]) ** (1.0 / n)
+                return bool((r[act] * rate ** (restart - n) > 10 * rtol * bn[act]).any())
             return False
 
         unread = None                         # a step issued and not read yet: (j, its event)
@@ -688,9 +689,10 @@ class DirectSolver:
             unread = (j, made)
             # The next step may be issued before this one is read where this one will not end the iteration: where
             # the last step's reduction, squared, would still leave a column 10x above the tolerance (a factor that
-            # converges in two or three steps never gets there: a step in vain costs more than its host part). The
+            # converges in two or three steps never gets there: a step in vain costs more than its host part), and
+            # where it would not be given up after this step even if the residuals stood still (they never grow). The
             # host's part of a step then runs beside the device's (stub filter, N = 2,553, 6 frequencies: 49 -> 44 ms).
-            if len(hist) >= 3 and j + 1 < restart:
+            if len(hist) >= 3 and j + 1 < restart and not ends(j + 1, hist[-1]):
                 ahead = hist[-1] * np.minimum(1.0, hist[-1] / np.maximum(hist[-2], SMALL)) ** 2
                 if (ahead[~done] > 10 * rtol * bn[~done]).any():
                     continue
