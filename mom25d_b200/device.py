@@ -171,7 +171,7 @@ class DeviceTables:
 
     def __init__(self, dg, f, single=False, stream=None):
         geo, st = dg.geo, dg.geo.st
-        self.f, self.w = f, 2 * np.pi * f
+        self.f, self.w, self.stream = f, 2 * np.pi * f, stream
         w = self.w
         s = stream_ptr(stream)
         pairs = geo.table_pairs()
@@ -268,6 +268,21 @@ class DeviceTables:
                                          P(self.scal32), P(self.scal32[npair:]), P(self.scal32[2 * npair:]),
                                          P(self.scal32[3 * npair:]), P(self.f32), P(self.f32[npair:]),
                                          P(self.f32[2 * npair:]), P(dg.tab), P(self.kind))
+
+    @property
+    def kr(self):
+        """The contour's nodes as a host array."""
+        return self._host_contour(self.d_kr)
+
+    @property
+    def dk(self):
+        """The contour's weights as a host array."""
+        return self._host_contour(self.d_dk)
+
+    def _host_contour(self, t):
+        if self.stream is not None:                        # (made there)
+            self.stream.synchronize()
+        return t.cpu().numpy()
 
     def host_dict(self, geo):
         """The tables as the reference core's tb dictionary (host copies), for checks."""

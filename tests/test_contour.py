@@ -1,4 +1,5 @@
-"""The host's Sommerfeld contour against the oracle's, for cut-offs K past the lifted part, on its end and before it."""
+"""The host's Sommerfeld contour against the oracle's, for cut-offs K past the lifted part, on its end and before it;
+and a frequency's tables' contour as host arrays."""
 import numpy as np
 import pytest
 
@@ -20,3 +21,14 @@ def test_host_contour(K, f):
     # breakpoints of m1 + n2 steps: a few ulp of the path's end in a node and in a weight
     tol = 16 * 2.0 ** -53 * max(K1, t1)
     assert np.abs(kr - kr0).max() <= tol and np.abs(dk - dk0).max() <= tol
+
+
+@pytest.mark.gpu
+def test_tables_have_their_contour():
+    from mom25d_b200 import board as B, device, geometry as G
+    geo = G.Geometry(B.microstrip_board(dmax=0.6e-3, length=10e-3))
+    tb = device.DeviceTables(device.DeviceGeometry(geo), 2.0e9)
+    kr, dk, K = green.sommerfeld_contour(2.0e9, geo.st, geo.rho_max)
+    tol = 16 * 2.0 ** -53 * K
+    assert tb.npts == len(tb.kr) == len(tb.dk) == len(kr)
+    assert np.abs(tb.kr - kr).max() <= tol and np.abs(tb.dk - dk).max() <= tol
