@@ -9,7 +9,8 @@
 //                  else k_panel_smem, a cooperative kernel with the rows in shared memory, or k_panel with the rows in
 //                  global memory and a bounded grid barrier a column.
 //   2. k_laswp     the panel's interchanges applied to the columns left and right of it.
-//   3. k_trsm      U12 = L11^-1 A12 (unit lower), one thread per column, L11 in shared memory.
+//   3. U12 = L11^-1 A12 (unit lower): k_trsm_outer on the critical path (a warp a column, with the interchanges of 2),
+//                  k_trsm64 on the far columns (a thread a column).
 //   4. trailing    A22 -= L21 U12: the complex SIMT GEMM below (FP64 / FP32), or the tensor-core 3xTF32 product
 //                  (umma.cu) for complex64 with tf32 on.
 #include <type_traits>
@@ -629,45 +630,11 @@ __global__ void __launch_bounds__(256) k_laswp_plan(R *A, long lda, int n, const
     else laswp_cols<R, 16, 1>(A, lda, P, a0, na, b0, nc, lane, wid, nw);
 }
 
-// A[k0 .. k0 + jb, c0 .. c1) = L11^-1 A[k0 .. k0 + jb, c0 .. c1), L11 = A[k0 .., k0 ..] unit lower (jb <= NB), in
-// shared memory; each thread one column
-// 64 columns a block of 256 threads: column c = tid % 64, rows split 4 ways (k % 4 == tid / 64); after row i is final
-// the block updates the rows below it (one barrier a row)
-template <typename R>
-__global__ void __launch_bounds__(256) k_trsm(R *A, long lda, int k0, int jb, long c0, long c1)
-{
-    typedef cpx<R> C;
-    extern __shared__ unsigned char sm_raw[];
-    C *L = reinterpret_cast<C *>(sm_raw);                  // L[k * NB + i] = L(k, i)
-    C *X = L + NB * NB;                                    // X[k * 64 + column]
-    for (int e = threadIdx.x; e < jb * jb; e += blockDim.x) {
-        int i = e / jb, k = e % jb;                        // column i, row k (coalesced)
-        L[k * NB + i] = ldc<R>(A, (size_t)(k0 + i) * lda + k0 + k);
-    }
-    const int cl = threadIdx.x & 63, g = threadIdx.x >> 6;
-    const long c = c0 + blockIdx.x * 64L + cl;
-    const bool live = c < c1;
-    for (int k = g; k < jb; k += 4) X[k * 64 + cl] = live ? ldc<R>(A, (size_t)c * lda + k0 + k) : mk<R>(0, 0);
-    __syncthreads();
-    for (int i = 0; i < jb - 1; ++i) {
-        const C xi = X[i * 64 + cl];
-        for (int k = i + 1 + ((g - (i + 1)) % 4 + 4) % 4; k < jb; k += 4) {
-            C x = X[k * 64 + cl];
-            cfms<R>(x, L[k * NB + i], xi);
-            X[k * 64 + cl] = x;
-        }
-        __syncthreads();
-    }
-    if (live)
-        for (int k = g; k < jb; k += 4) stc<R>(A, (size_t)c * lda + k0 + k, X[k * 64 + cl]);
-}
-
-
-// The same for a full panel (jb = NB = 64) without a barrier inside the substitution: a warp solves 32
-// columns, one a lane, the lane's column in registers (64 complex), L11 in shared memory read as broadcasts. The
-// columns are staged through shared memory (a column's stride NB + 1: the lanes' reads of their own columns fall in
-// different banks) so that every global load and store is a warp's 256 contiguous bytes. The arithmetic and its
-// order are those of k_trsm (row i's multiple subtracted from the rows below, i ascending).
+// A[k0 .. k0 + NB, c0 .. c1) = L11^-1 A[k0 .. k0 + NB, c0 .. c1), L11 = A[k0 .., k0 ..] unit lower: a panel's U12 on the
+// far columns. A warp solves 32 columns, one a lane, 16 rows at a time in registers, L11 in shared memory read as
+// broadcasts. The columns are staged through shared memory (a column's stride NB + 1: the lanes' reads of their own
+// columns fall in different banks) so that every global load and store is a warp's 256 contiguous bytes. Row i's
+// multiple is subtracted from the rows below, i ascending.
 template <typename R, int T64_WARPS>
 __global__ void __launch_bounds__(32 * T64_WARPS) k_trsm64(R *A, long lda, int k0, long c0, long c1)
 {
@@ -1901,7 +1868,8 @@ extern "C" int m25_set_lu_tuning(int single, const int *h_n, const int *h_nb2, c
     return M25_OK;
 }
 
-// The parameters at size n (complex64 when single): the table's entry nearest in log n, else the defaults; M25_NB2 and M25_PANEL_BLOCKS in the environment override both.
+// The parameters at size n (complex64 when single): the table's entry nearest in log n, else the defaults; M25_NB2 and
+// M25_PANEL_BLOCKS in the environment override both.
 extern "C" int m25_get_lu_tuning(int n, int single, int *nb2, int *blocks)
 {
     int G = sm_count();
@@ -1968,8 +1936,6 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
     M25_CHECK(cudaStreamWaitEvent(Lo, ev_start, 0));
     M25_CHECK(cudaMemsetAsync(ipiv, 0xff, sizeof(int) * (size_t)n, H));      // -1 until the panel sets it
     M25_CHECK(cudaMemsetAsync(pw.ll_cand, 0, ll_bytes, H));         // flags 0: no column's (they are column + 1)
-    const size_t trsm_smem = sizeof(cpx<R>) * (NB * NB + NB * 64);
-    M25_CHECK(cudaFuncSetAttribute(k_trsm<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem));
     M25_CHECK(cudaFuncSetAttribute(k_trsm64<R, t64_warps<R>()>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)t64_smem<R>()));
     M25_CHECK(cudaFuncSetAttribute(k_trsm_outer<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)to_smem<R>()));
@@ -2026,18 +1992,13 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
         M25_LAUNCH_CHECK("k_laswp_plan");
         return M25_OK;
     };
-    // U12 rows k0 .. k0 + jb of the columns [c0, c1), their interchanges applied before
-    auto trsm = [&](int k0, int jb, long c0, long c1, cudaStream_t cs) -> int {
+    // U12 rows k0 .. k0 + NB of the columns [c0, c1), their interchanges applied before
+    auto trsm = [&](int k0, long c0, long c1, cudaStream_t cs) -> int {
         if (c1 <= c0) return M25_OK;
-        if (jb == NB) {
-            const long per = 32L * t64_warps<R>();
-            k_trsm64<R, t64_warps<R>()><<<(unsigned)((c1 - c0 + per - 1) / per), (unsigned)per, t64_smem<R>(), cs>>>(
-                A, lda, k0, c0, c1);
-            M25_LAUNCH_CHECK("k_trsm64");
-            return M25_OK;
-        }
-        k_trsm<R><<<(c1 - c0 + 63) / 64, 256, trsm_smem, cs>>>(A, lda, k0, jb, c0, c1);
-        M25_LAUNCH_CHECK("k_trsm");
+        const long per = 32L * t64_warps<R>();
+        k_trsm64<R, t64_warps<R>()><<<(unsigned)((c1 - c0 + per - 1) / per), (unsigned)per, t64_smem<R>(), cs>>>(
+            A, lda, k0, c0, c1);
+        M25_LAUNCH_CHECK("k_trsm64");
         return M25_OK;
     };
     // U12 of the panel [K0, K0 + JB) (a panel, or the whole outer panel) on the columns [c0, c1), its interchanges
@@ -2168,10 +2129,9 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
         if ((rc = laswp(K0, JB, 0, K0, KE2, n, 0, 1, Lo))) return rc;      // (one launch for both)
         next_pending = false;
         if (KE2 < n) {
-            for (int k0 = K0; k0 < KE; k0 += NB) {
-                const int jb = std::min(NB, KE - k0);
-                if ((rc = trsm(k0, jb, KE2, n, Lo))) return rc;
-                if ((rc = gemm(k0 + jb, KE - k0 - jb, KE2, n - KE2, k0, jb, true, Lo))) return rc;
+            for (int k0 = K0; k0 < KE; k0 += NB) {                        // (whole panels: only the last block has less)
+                if ((rc = trsm(k0, KE2, n, Lo))) return rc;
+                if ((rc = gemm(k0 + NB, KE - k0 - NB, KE2, n - KE2, k0, NB, true, Lo))) return rc;
             }
             if ((rc = gemm(KE, n - KE, KE2, KE3 - KE2, K0, JB, tc, Lo))) return rc;   // block k + 2's columns
             M25_CHECK(cudaEventRecord(ev_next, Lo));
