@@ -288,9 +288,13 @@ def run_gpu(args, rank, world):
     cold()
     gc.collect()
     gc.disable()
+    e2e_path, e2e_s = [], []
     e0.record(stream)
     for i in range(args.steps):
+        t = time.perf_counter()
         sim.sparams(mine[i % len(mine)])
+        e2e_s.append(time.perf_counter() - t)
+        e2e_path.append(ds.last_path)
     e1.record(stream)
     torch.cuda.synchronize()
     gc.enable()
@@ -341,7 +345,8 @@ def run_gpu(args, rank, world):
         "kept_lus_max": int(ds._keep_max()),
         "phases_ms_per_step": phases,
         "e2e": {"value": round(e2e, 4), "unit": "freq-solves/s", "h2d_bytes_per_step": bytes_h2d,
-                "d2h_bytes_per_step": bytes_d2h},
+                "d2h_bytes_per_step": bytes_d2h,
+                "per_step": {"path": e2e_path, "ms": [round(1000 * x, 2) for x in e2e_s]}},
         "gpu_launches": int(launches),
         "roofline": {"kernel": "complex64 LU with 3xTF32 tcgen05 updates (m25_getrf), 8/3 N^3 flops a factorisation",
                      "bound": "tensor", "achieved": round(achieved, 2), "peak": tensor_peak, "unit": "TFLOP/s",
@@ -397,18 +402,19 @@ def time_solve_pair(ds, k, reps=10):
     return statistics.median(times)
 
 
-# FP64 flops of the fill per Z entry (edge tiles: 56 an entry + 30 a kernel evaluation, 0.95 evaluations an entry)
-FILL_FLOPS_PER_ENTRY = 56 + 30 * 0.95
+# FP64 flops of the fill per Z entry. Z is symmetric and an entry and its mirror image are formed once: four triangle
+# pairs of 12 (two weights, four multiply-adds) and 6 for the two scaled sums, and 0.95 kernel evaluations of 30.
+FILL_FLOPS_PER_ENTRY = (4 * 12 + 6 + 0.95 * 30) / 2
 FP64_PEAK_TFLOPS = 36.6                  # a loop of independent FP64 FMAs over 148 x 8 CTAs of 256 threads, this B200
 
 
 def fill_roofline(geo, fill_ms):
-    """The fill's roofline (far fill + near correction, double precision, once a step): Ne^2 entries x 84.5 flops
+    """The fill's roofline (far fill + near correction, double precision, once a step): Ne^2 entries x 41.25 flops
     against the FP64 FMA rate measured on this pool's B200 (no FP64 figure in MEASURED_PEAKS.json)."""
     if not fill_ms:
         return None
     achieved = geo.Ne ** 2 * FILL_FLOPS_PER_ENTRY / (fill_ms / 1000.0) / 1e12
-    return {"kernel": "far fill + near correction in FP64 (m25_fill_far, m25_near), Ne^2 x 84.5 flops a fill",
+    return {"kernel": "far fill + near correction in FP64 (m25_fill_far, m25_near), Ne^2 x 41.25 flops a fill",
             "bound": "fp64", "achieved": round(achieved, 2), "peak": FP64_PEAK_TFLOPS, "unit": "TFLOP/s",
             "frac": round(achieved / FP64_PEAK_TFLOPS, 4), "ms": fill_ms,
             "peak_source": "FP64 FMA loop measured on this pool's B200 (not in MEASURED_PEAKS.json)"}
