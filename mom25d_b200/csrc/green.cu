@@ -719,11 +719,12 @@ extern "C" int m25_spline_uniform(const double *d_x, const double *d_y, int ns, 
 {
     M25_REQUIRE(n >= 4 && ns >= 1 && nfine >= 2, "m25_spline_uniform: n >= 4 points");
     size_t smem = sizeof(zd) * (4 * (size_t)(n - 1) + n) + sizeof(double) * n;
-    M25_REQUIRE(smem <= 200 * 1024, "m25_spline_uniform: too many knots");
+    constexpr int smem_max = 200 * 1024;               // (the limit of every call: it is the process's, not the call's)
+    M25_REQUIRE(smem <= smem_max, "m25_spline_uniform: too many knots");
     const dim3 grid(ns, std::min(16, (nfine + 511) / 512));            // (2 points a thread at 8,192)
     auto go = [&](auto kernel, auto *out) -> int {
         if (smem > 48 * 1024)
-            M25_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            M25_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
         kernel<<<grid, 256, smem, S(stream)>>>(d_x, d_y, n, dx, nfine, out, out_stride, out_offset_elems, out_interleave);
         return M25_OK;
     };

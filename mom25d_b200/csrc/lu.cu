@@ -2157,6 +2157,11 @@ extern "C" int m25_getrf(void *d_A, long lda, int n, int *d_ipiv, int single, in
     return M25_OK;
 }
 
+// Limits of the dynamic shared memory of kernels whose need grows with n. A kernel's limit is one setting of the whole
+// process: it is always set to the largest, never to a call's own need, which another thread's smaller call could set
+// back between this call's setting and its launch.
+constexpr int PERM_SMEM_MAX = 200 * 1024, TRSV_SMEM_MAX = 200 * 1024;
+
 template <typename R>
 static size_t aux_layout(int n, size_t *off_inv, size_t *off_perm, size_t *off_w, size_t *off_flags = nullptr)
 {
@@ -2212,8 +2217,8 @@ static int getrs_prepare_impl(const R *A, long lda, int n, const int *ipiv, unsi
     const size_t basic = sb_offset(n, single);
     if (use_sb) M25_REQUIRE(aux_bytes >= basic + m25_sb_bytes(n, single), "m25_getrs_prepare: aux buffer too small");
     const int nb = (n + TB - 1) / TB;
-    M25_REQUIRE(sizeof(int) * (size_t)n <= 200 * 1024, "m25_getrs_prepare: n above 51200");
-    M25_CHECK(cudaFuncSetAttribute(k_perm_from_ipiv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(int) * n)));
+    M25_REQUIRE(sizeof(int) * (size_t)n <= PERM_SMEM_MAX, "m25_getrs_prepare: n above 51200");
+    M25_CHECK(cudaFuncSetAttribute(k_perm_from_ipiv, cudaFuncAttributeMaxDynamicSharedMemorySize, PERM_SMEM_MAX));
     // the plans where the block inverses go afterwards (64 KB or more for every 64 rows), the flag where the solves'
     // epoch counter is (zeroed below)
     static_assert(sizeof(PermChunk) <= 2 * TB * TB * sizeof(cpx<R>), "room for the plans");
@@ -2262,8 +2267,8 @@ static int getrs_aux_impl(const R *A, long lda, int n, unsigned char *aux, R *B,
     // 4.8 / 5.3 / 6.6 ms with 100 / 74 / 59, each owning more consecutive blocks)
     const int G = std::max(1, std::min(sm_count(), nb));
     const size_t sm = trsv_smem<R>(n, G);
-    M25_REQUIRE(sm <= 200 * 1024, "m25_getrs_aux: n too large for the persistent solve");
-    M25_CHECK(cudaFuncSetAttribute(k_trsv_persistent<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    M25_REQUIRE(sm <= TRSV_SMEM_MAX, "m25_getrs_aux: n too large for the persistent solve");
+    M25_CHECK(cudaFuncSetAttribute(k_trsv_persistent<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, TRSV_SMEM_MAX));
     k_bump_epoch<<<1, 1, 0, s>>>(epoch);                                    // this call's flag value
     M25_LAUNCH_CHECK("k_bump_epoch");
     TrsvArgs<R> fa{A, lda, n, nb, inv, B, W1, nrhs, 0, flags, epoch, err};          // U^T y = b: B -> W1
@@ -2272,7 +2277,8 @@ static int getrs_aux_impl(const R *A, long lda, int n, unsigned char *aux, R *B,
     int smem_optin = 0, dev = 0;
     M25_CHECK(cudaGetDevice(&dev));
     M25_CHECK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    if (per <= TRSV_MAXPER && trsv_pipe_smem<R>(per) + 256 <= (size_t)smem_optin) {
+    const int pipe_max = smem_optin - 256;                                 // less the kernel's static shared memory
+    if (per <= TRSV_MAXPER && trsv_pipe_smem<R>(per) <= (size_t)pipe_max) {
         // the factor tiles through shared memory (cp.async, 16-byte pieces where rows allow); the kernel for the
         // smallest compile-time column count >= nrhs
         const size_t psm = trsv_pipe_smem<R>(per);
@@ -2280,7 +2286,7 @@ static int getrs_aux_impl(const R *A, long lda, int n, unsigned char *aux, R *B,
         const void *kf = nrhs <= 1 ? (const void *)k_trsv_pipe<R, 1> : nrhs <= 2 ? (const void *)k_trsv_pipe<R, 2> :
                          nrhs <= 4 ? (const void *)k_trsv_pipe<R, 4> : nrhs <= 8 ? (const void *)k_trsv_pipe<R, 8> :
                          (const void *)k_trsv_pipe<R, 16>;
-        M25_CHECK(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+        M25_CHECK(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, pipe_max));
         void *fargs[] = {&fa, &vec16};
         M25_CHECK(cudaLaunchCooperativeKernel(kf, dim3(G), dim3(TRSV_NT), fargs, psm, s));
         m25_note_launch();
