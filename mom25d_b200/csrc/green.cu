@@ -364,9 +364,12 @@ __global__ void k_contour(double t1, double alpha, double K, double wid2, int m1
 // ---- Hankel transform (via.py:90-108): out[s, i] = (1/2pi) sum_k J0(rho_i kr_k) W[s, k] kr_k dk_k -------------------
 // A cluster of HB blocks a radius: the contour split over their threads (J0 of a real argument: the CUDA math library's
 // j0; on the lifted part the complex series above), a block reduction per spectrum, then the blocks' sums added in
-// order through distributed shared memory. Bound by the FP64 Bessel values. HB = 4 where the radii alone do not fill
-// the SMs (a via group's distances, 1 to 64: 51 -> 20 us a launch), 1 where they do (the tables' 260 and 200: 88 us,
-// with 4 blocks 100).
+// order through distributed shared memory. Bound by the FP64 Bessel values. HB = 4 where all clusters run at once, two
+// blocks an SM (a via group's distances, 1 to 64 of them: 51 -> 20 us a launch), else 1 (the tables' 260 and 200 radii:
+// 88 us, with 4 blocks 100). Clusters of four do not fill every group of SMs: on 148 SMs 70 of them still do, 74 do not,
+// so the line is drawn at 64. Measured with 1 / 4 blocks: 1,500 points and 4, 8, 16 spectra, 64 radii 36.5 / 35.6,
+// 36.8 / 34.8, 38.9 / 36.7 us, 100 radii 36.8 / 37.8, 37.1 / 53.6, 38.9 / 56.5, 148 radii 36.5 / 53.3, 37.5 / 62.0,
+// 40.0 / 66.1; 6,000 points and 8 spectra, 64 radii 65.6 / 41.1, 100 66.0 / 63.8, 148 66.1 / 78.2.
 // RAW: the bare sum over real kr (hankel_real, mom25d_core.cpp:1430-1454): out[s, i] = sum_k J0(rho_i kr_k) W[s, k],
 // kr_ real f64[npts], no dk, no 1 / 2 pi.
 template <int NS, int HB, bool RAW = false>
@@ -684,9 +687,12 @@ template <bool RAW>
 static void hankel_launch(const double *kr, const double *dk, int npts, const double *W, int ns, const double *rho,
                           double *out, int nr, cudaStream_t s)
 {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        (void)cudaGetLastError();
     auto go = [&](auto nsm) {
         constexpr int NS = decltype(nsm)::value;
-        if (nr > 148) k_hankel<NS, 1, RAW><<<nr, 256, 0, s>>>(kr, dk, npts, W, ns, rho, out, nr);
+        if (16 * (long)nr > 7 * (long)sms) k_hankel<NS, 1, RAW><<<nr, 256, 0, s>>>(kr, dk, npts, W, ns, rho, out, nr);
         else k_hankel<NS, 4, RAW><<<dim3(nr, 4), 256, 0, s>>>(kr, dk, npts, W, ns, rho, out, nr);
     };
     if (ns <= 4) go(std::integral_constant<int, 4>());

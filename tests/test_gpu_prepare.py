@@ -131,3 +131,29 @@ def test_hankel(ns, npts, nr):
     got = core.hankel_real(rho, kr.real.copy(), W)
     want, size = W @ j0(rho[:, None] * kr.real).T, np.abs(W).sum(1)[:, None]
     assert (np.abs(got - want) <= (2e-13 + npts * 2.0 ** -52) * size).all()
+
+
+@pytest.mark.parametrize('nr', [1, 64, 65, 100, 148])
+@pytest.mark.parametrize('ns,npts', [(4, 1025), (16, 700)])
+def test_hankel_blocks_a_radius(ns, npts, nr):
+    """Up to 64 radii (7/16 of the SMs) are summed by four blocks each, more by one: from there on a radius's sum is that
+    of a call with many radii, bit for bit; below it is, to rounding."""
+    from mom25d_b200 import _lib
+    from mom25d_b200._lib import P, check, lib
+    rng = np.random.default_rng(nr)
+    c = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)
+    kr, dk, W = np.linspace(1.0, 900.0, npts) + 0j, c(npts), c(ns, npts)
+    rho = np.linspace(1e-4, 0.07, 260)
+    d_kr, d_dk, d_W = (_lib.dev(v) for v in (kr, dk, W))
+
+    def sums(r):
+        d_rho, out = _lib.dev(r), torch.empty((ns, len(r)), dtype=torch.complex128, device='cuda')
+        check(lib().m25_hankel(P(d_kr), P(d_dk), npts, P(d_W), ns, P(d_rho), len(r), P(out), _lib.stream_ptr()), 'm25_hankel')
+        _lib.sync_check()
+        return out.cpu().numpy()
+    got, many = sums(rho[:nr]), sums(rho)[:, :nr]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if 16 * nr > 7 * sms:
+        assert np.array_equal(got, many)
+    size = np.abs(W) @ np.abs(kr * dk) / (2 * np.pi)       # |J0| <= 1, npts additions in either order
+    assert (np.abs(got - many) <= npts * 2.0 ** -52 * size[:, None]).all()
