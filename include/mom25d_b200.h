@@ -256,9 +256,10 @@ int m25_getrf(void *d_A, long lda, int n, int *d_ipiv, int single, int tf32, voi
 /* The LU's tile parameters by matrix size (no counterpart in the reference: LAPACK picks its own blocking): a
  * table for complex64 (single = 1) and one for complex128 factorisations, up to 32 entries each (n, outer panel
  * width nb2 = 64..256 in steps of 64, cooperative panel blocks), as the autotuner (mom25d_b200/tune.py) finds them
- * on this GPU; a factorisation of size n takes the entry nearest to n in log n. count 0 restores the defaults
+ * on this GPU; a factorisation of size n takes the panel blocks of the entry nearest to n in log n, and for each outer
+ * panel the width of the entry nearest to the size that is left to factor. count 0 restores the defaults
  * (256, min(SMs, 32)). The environment variables M25_NB2 and M25_PANEL_BLOCKS override both.
- * m25_get_lu_tuning: what a factorisation of size n uses. */
+ * m25_get_lu_tuning: the entry of size n. */
 int m25_set_lu_tuning(int single, const int *h_n, const int *h_nb2, const int *h_blocks, int count);
 int m25_get_lu_tuning(int n, int single, int *nb2, int *blocks);
 /* Solves Z X = B with the factor of Z^T (lu_solve(..., trans=1)); B (row-major n x nrhs, complex in the factor's

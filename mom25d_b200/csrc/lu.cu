@@ -1962,10 +1962,10 @@ static int getrf_impl(R *A, long lda, int n, int *ipiv, int tf32, void *work, si
     m25_get_lu_tuning(n, sizeof(R) == 4, nullptr, &gmax);            // default
     // Columns of an outer block: the table's width for a matrix of the size that is left there. A wide block has fewer
     // and deeper updates of the far columns; a narrow one keeps the critical path short, which decides where those
-    // updates are done before the panels are (the committed table's lines: 64 columns below 2,828 left, 128 below 5,000
-    // in complex64 and 5,477 in complex128, 256 above). Measured, one width throughout (complex64 256; complex128 128,
-    // at 9,601 256) against this: complex64 n = 1,000 2.26 / 2.03 ms, 2,921 6.82 / 6.15, 4,977 13.1 / 12.1, 7,000
-    // 20.9 / 19.3; complex128 1,000 2.78 / 2.58, 2,921 8.87 / 8.17, 5,000 21.1 / 20.6, 7,000 44.4 / 43.3.
+    // updates are done before the panels are (the committed table's lines: 64 columns below 2,828 left, 128 below 5,099
+    // in complex64 and 5,477 in complex128, 256 above). Measured, ms with 64 / 128 / 256 columns down to the line below:
+    // complex128 n = 1,000 2.75 / 2.97 / 3.03, 2,828 8.20 / 8.74 / 9.29, 4,000 14.07 / 13.45 / 14.16, 7,500 53.8 / 50.8 /
+    // 49.9; complex64 2.20 / 2.20 / 2.19, 6.37 / 6.44 / 6.50, 10.4 / 9.4 / 9.5 (6,250: 128 / 256 17.2 / 17.1).
     const std::unique_ptr<int[]> start(new (std::nothrow) int[n / NB + 1]);    // first columns, read once (another
     M25_REQUIRE(start, "m25_getrf: out of host memory");                       // thread may set the table)
     int nblk = 0;

@@ -1,7 +1,7 @@
 """
 mom25d_b200.tune - the autotuner of the LU's tile parameters, and timings of the hot path's kernels on this GPU.
 
-    python -m mom25d_b200.tune --autotune [--sizes 2000 5000 10000 20000 40000] [--write]
+    python -m mom25d_b200.tune --autotune [--sizes 1000 2000 ... 40000] [--write]
     python -m mom25d_b200.tune --lu 8192 [--single] [--tf32] [--reps 3]     # the LU alone, CUDA events
     python -m mom25d_b200.tune --update 4096 4096 256                        # the tensor-core trailing update
     python -m mom25d_b200.tune --solve 18788 [--single]                      # the triangular solves, 8 columns
@@ -10,19 +10,28 @@ mom25d_b200.tune - the autotuner of the LU's tile parameters, and timings of the
 Times are CUDA-event measurements on the launching stream after a warm-up, the matrix a random complex one with a
 dominant diagonal (pivots away from it as well).
 
-The autotuner times the LU at each size over its host-side parameters and keeps the fastest: for the complex64
-LU with tensor-core updates (the mixed path's factorisation) the number of CTAs of the cooperative panel kernel
-(16 to 64), with an outer panel width of 256 columns, or of 64 where every update is in FP32 - the widths between
-leave more of the factor's updates to 3xTF32 instead of FP32 and cost the factor its use as a preconditioner at the
-low-frequency end (measured on the routed board: with 128, the fresh factor at 0.67 GHz no longer converged). With at
-most 8,000 rows left the next block's columns too are updated in FP32, which makes up for a narrower block: the
-committed file's 128 columns at 4,000 are of that kind (n = 4,977: residual of the factor 0.9e-4 against 1.7e-4 with
-256 and the next block's columns in 3xTF32) and are entered by hand. For the complex128 LU (the drop-in) both the outer
-panel width (64 / 128 / 192 / 256) and the panel CTAs are searched. The winners per size go into TUNING_FILE
-({"device", "sms", "complex64": [{"n", "nb2", "blocks", "ms"}], "complex128": [...]}), which the library reads at
-load (_lib.apply_tuning -> m25_set_lu_tuning): a factorisation takes the panel CTAs of the entry nearest its size, and
-for each outer panel the width of the entry nearest the size that is left to factor. The tensor-core kernel's stage
-count is a compile-time choice (two stages, two CTAs an SM) and is not searched.
+The autotuner fills the LU's table from the smallest size up. A factorisation takes, for each outer block, the width of
+the entry nearest (in log n) to the size that is left, so the entry of a size decides the blocks down to the line with
+the entry below (their geometric mean), and what is left below that line is factored as the entries found before say:
+each candidate is timed as the whole table it would make, the candidates of a size in turn, several times over. The sizes
+are therefore where the widths may change: with the default ones (SIZES) at 1,414, 2,828, 5,099 and 8,062 rows left
+and above in complex64, at 1,414, 2,828, 5,477, 8,660 and above in complex128.
+
+Searched is the outer width; the CTAs of the cooperative panel kernel (16 to 64) only with M25_PANEL_CLUSTER=0 (the panels
+that have more rows than a thread-block cluster takes need more CTAs than that for their shared memory). Widths: 64 to
+256 for the complex128 LU (the drop-in); of times within TIE the widest. For the complex64 LU with tensor-core updates (the mixed path's factorisation) 256, or 64,
+where every update is in FP32: the widths between leave more of the factor's updates to 3xTF32 instead of FP32 and cost
+the factor its use as a preconditioner at the low-frequency end (measured on the routed board: with 128, the fresh
+factor at 0.67 GHz no longer converged). With at most FP32_ROWS rows left the next block's columns too are updated in
+FP32, which makes up for it (n = 4,977: residual of the factor 0.9e-4 with 128 against 1.7e-4 with 256 and the next
+block's columns in 3xTF32): 128 is searched for the entries whose lines lie below that. The widths then differ little (64,
+128, 256: 2.20, 2.20, 2.19 ms at 1,000; 4.47, 4.46, 4.55 at 2,000; 10.38, 9.41, 9.49 at 4,000; 1% either way on another
+GPU), and of times within TIE the narrowest is taken, which leaves more of the factor to FP32. (128 up to 6,847 rows left
+was measured too: 17.30 against 17.25 ms at 6,250, 33.5 against 33.0 at 9,601.)
+
+The winners go into TUNING_FILE ({"device", "sms", "complex64": [{"n", "nb2", "blocks", "ms"}], "complex128": [...]}; ms:
+the LU of that size with the table), which the library reads at load (_lib.apply_tuning -> m25_set_lu_tuning). The
+tensor-core kernel's stage count is a compile-time choice (two stages, two CTAs an SM) and is not searched.
 """
 import os
 import argparse
@@ -47,8 +56,23 @@ def random_matrix(n, dtype, seed=0):
 
 
 TUNING_FILE = os.path.join(os.path.dirname(os.path.abspath(__file__)), 'tuning_b200.json')
-GRIDS = {True: [(256, bl) for bl in (16, 24, 32, 48, 64)] + [(64, 32)],
-         False: [(b2, bl) for b2 in (64, 128, 192, 256) for bl in (16, 32, 48)]}
+SIZES = {True: [1000, 2000, 4000, 6500, 10000, 20000, 40000], False: [1000, 2000, 4000, 7500, 10000, 20000]}
+FP32_ROWS = 8000               # lu.cu WIN_ROWS: rows left at which the next block's columns go to FP32 (complex64)
+TIE = {True: 0.015, False: 0.005}      # times within this of the shortest count as equal
+
+
+def candidates(n, above, single):
+    """The (width, panel CTAs) tried at size n when the next larger entry is at `above` (None: there is none), of equal
+    ones the preferred first."""
+    if single:
+        line = (n * above) ** 0.5 if above else float('inf')
+        widths = (64, 128, 256) if line <= FP32_ROWS else (64, 256)
+    else:
+        widths = (256, 192, 128, 64)
+    blocks = (32 if single or n < 4000 else 16,)
+    if os.environ.get('M25_PANEL_CLUSTER') == '0':
+        blocks = (16, 24, 32, 48, 64) if n <= 20000 else (32, 48)
+    return [(w, b) for w in widths for b in blocks if w > 64 or n <= 20000]    # (above, 64 is seconds a try)
 
 
 def set_table(entries, single=True):
@@ -58,25 +82,25 @@ def set_table(entries, single=True):
 
 
 def autotune(sizes, single=True, reps=2, log=print):
-    """The fastest (nb2, blocks) per size for the complex64 (tensor-core) or complex128 LU:
-    [{n, nb2, blocks, ms, grid: {"nb2/blocks": ms}}]."""
-    out = []
-    for n in sizes:
-        grid = GRIDS[single]
-        if n > 30000:                                     # (the largest size: a coarser grid, each LU is seconds)
-            grid = [g for g in grid if g[0] > 64 and g[1] in (32, 48)][:4]
-        times = {}
-        for b2, bl in grid:
-            set_table([(1, b2, bl)], single)
-            times[f"{b2}/{bl}"] = time_lu(n, single=single, tf32=single, reps=reps)['ms']
-        best = min(times, key=times.get)
-        b2, bl = map(int, best.split('/'))
-        out.append(dict(n=int(n), nb2=b2, blocks=bl, ms=round(times[best], 2), grid={k: round(v, 2) for k, v in
-                                                                                     times.items()}))
+    """The table of the complex64 (tensor-core) or complex128 LU, left set in the library: [{n, nb2, blocks, ms, grid:
+    {"nb2/blocks": ms}}] by rising n."""
+    out, sizes = [], sorted(sizes)
+    entry = lambda e: (e['n'], e['nb2'], e['blocks'])
+    for i, n in enumerate(sizes):
+        above = sizes[i + 1] if i + 1 < len(sizes) else None
+        times = {c: [] for c in candidates(n, above, single)}
+        for _ in range(reps if n > 10000 else 3 * reps):
+            for b2, bl in times:
+                set_table([entry(e) for e in out] + [(int(n), b2, bl)], single)
+                times[b2, bl].append(time_lu(n, single=single, tf32=single, reps=1 if n > 10000 else 5)['ms'])
+        times = {c: float(np.median(t)) for c, t in times.items()}
+        b2, bl = next(c for c in times if times[c] <= (1 + TIE[single]) * min(times.values()))
+        out.append(dict(n=int(n), nb2=b2, blocks=bl, ms=round(times[b2, bl], 2),
+                        grid={f'{w}/{b}': round(v, 2) for (w, b), v in times.items()}))
         if log:
-            log(f"{'complex64' if single else 'complex128'} n={n}: nb2 {b2}, panel blocks {bl}: {times[best]:.1f} ms "
-                f"(default 256/32: {times.get('256/32', float('nan')):.1f} ms)")
-    set_table([(e['n'], e['nb2'], e['blocks']) for e in out], single)
+            log(f"{'complex64' if single else 'complex128'} n={n}: nb2 {b2}, panel blocks {bl}: {times[b2, bl]:.2f} ms "
+                f"of {out[-1]['grid']}")
+    set_table([entry(e) for e in out], single)
     return out
 
 
@@ -197,13 +221,13 @@ def main():
     ap.add_argument('--tf32', action='store_true')
     ap.add_argument('--reps', type=int, default=3)
     ap.add_argument('--autotune', action='store_true')
-    ap.add_argument('--sizes', type=int, nargs='+', default=[2000, 5000, 10000, 20000, 40000])
+    ap.add_argument('--sizes', type=int, nargs='+', default=None)
     ap.add_argument('--write', action='store_true', help='write the autotuner\'s table to ' + TUNING_FILE)
     a = ap.parse_args()
     _lib.require_cuda()
     if a.autotune:
-        c64 = autotune(a.sizes, single=True, reps=max(1, min(a.reps, 2)))
-        c128 = autotune([n for n in a.sizes if n <= 20000], single=False, reps=1)
+        c64 = autotune(a.sizes or SIZES[True], single=True, reps=max(1, min(a.reps, 2)))
+        c128 = autotune([n for n in a.sizes or SIZES[False] if n <= 20000], single=False, reps=1)
         print(json.dumps(dict(complex64=c64, complex128=c128)))
         if a.write:
             print('wrote', write_tuning(c64, c128))

@@ -50,3 +50,54 @@ def test_tuning_file_is_applied(tmp_path):
         L.m25_set_lu_tuning(1, None, None, None, 0)
         L.m25_set_lu_tuning(0, None, None, None, 0)
         _lib.apply_tuning(L)                               # back to the committed table, if any
+
+
+def _lu_model(lines, tried):
+    """A stand-in for tune.time_lu: a factorisation's outer blocks are walked as m25_getrf walks them, each at the width
+    the library's table has for the size left; a row costs 1 at the best width there (lines: {width: rows left above
+    which it is the best}), more the further its width is from that."""
+    def time_lu(n, single=False, tf32=False, reps=3):
+        ms, left = 0.0, n
+        while left > 0:
+            w = _get(_lib.lib(), left, int(single))[0]
+            best = max((b for b in lines if left > lines[b]), key=lambda b: lines[b])
+            ms += min(w, left) * (1 + abs(w - best) / 64) * 1e-3
+            tried.append((single, left, w))
+            left -= w
+        return dict(ms=ms)
+    return time_lu
+
+
+@pytest.mark.parametrize('single,lines,want', [
+    (True, {64: 0, 128: 2828, 256: 5000}, {500: 64, 2700: 64, 2900: 128, 4900: 128, 5100: 256, 18788: 256}),
+    (False, {64: 0, 128: 2828, 256: 5477}, {500: 64, 2700: 64, 2900: 128, 5400: 128, 5600: 256, 18788: 256}),
+    (False, {128: 0, 192: 5477, 256: 8660}, {500: 128, 5400: 128, 5600: 192, 8600: 192, 8700: 256, 18788: 256})])
+def test_autotuner_finds_the_lines(single, lines, want, monkeypatch):
+    """The autotuner times the tables a factorisation uses: with costs that change at the lines between its sizes it
+    finds the widths on both sides of each, the 128 columns of the complex64 table among them."""
+    from mom25d_b200 import tune
+    monkeypatch.delenv('M25_NB2', raising=False)
+    monkeypatch.delenv('M25_PANEL_BLOCKS', raising=False)
+    tried = []
+    monkeypatch.setattr(tune, 'time_lu', _lu_model(lines, tried))
+    L = _lib.lib()
+    try:
+        out = tune.autotune(tune.SIZES[single], single=single, log=None)
+        assert {n: _get(L, n, int(single))[0] for n in want} == want
+        assert all(set(e) >= {'n', 'nb2', 'blocks', 'ms'} for e in out)
+        if single:                                         # 3xTF32 on the next block's columns: 64 or 256 only
+            assert all(w in (64, 256) for s, left, w in tried if left > tune.FP32_ROWS)
+    finally:
+        _lib.apply_tuning(L)
+
+
+def test_committed_table():
+    """The committed table is of the autotuner's own form: its sizes, its candidates, a time each."""
+    from mom25d_b200 import tune
+    doc = json.load(open(tune.TUNING_FILE))
+    for key, single in (('complex64', True), ('complex128', False)):
+        es = doc[key]
+        ns = [e['n'] for e in es]
+        assert ns == tune.SIZES[single] and all(e['ms'] > 0 for e in es)
+        for e, above in zip(es, ns[1:] + [None]):
+            assert (e['nb2'], e['blocks']) in tune.candidates(e['n'], above, single)
