@@ -9,7 +9,7 @@ The workload is the stub filter board (board.stub_filter_board: three layers 0.2
 linspace(fmin, fmax, freqs).
 
   - batched: the Green tables of every frequency are built and kept on the device, and the far part of every
-    frequency's double Z is filled by one launch (m25_fill_far_multi, grid z = frequency; in chunks where the
+    frequency's double Z is filled by one launch (m25_fill_far_multi, grid y = frequency; in chunks where the
     matrices of all frequencies would not fit); then all frequencies are present at the start and go through the
     serving loop (serve.Server), each with its prefilled Z: each slot has its own CUDA stream, host thread and
     solver, which adds the near field and via border, factors and refines, so one frequency's panel

@@ -209,8 +209,9 @@ __device__ __forceinline__ void fill_far_tile(R *Z, long ld, const m25_mesh &g, 
     }
 }
 
-// four CTAs an SM (64 registers; 88 let two): the tile's phases end in barriers, and the other CTAs' warps fill
-// those stalls
+// Four CTAs an SM: the tile's phases end in barriers, and the other CTAs' warps fill those stalls. The 64 registers that
+// leaves spill (68 bytes a thread stored in double; 80, three CTAs, still 44). Four / three CTAs: double, Ne = 8,213
+// 0.913 / 0.917 ms, 15,706 3.37 / 3.33; single 0.675 / 0.736 and 2.44 / 2.66.
 template <typename R, typename TB>
 __global__ void __launch_bounds__(256, 4) k_fill_far(R *Z, long ld, m25_mesh g, TB tb, double w)
 {

@@ -557,11 +557,13 @@ int m25_panel_cluster_rows(int single, int cl) { return cl * 512 * (single ? 4 :
 // Factors the panel of columns k0 .. k0 + jb (jb <= 64), rows k0 .. n, on a cluster of at most cl CTAs.
 //
 // CTAs: one for every 128 rows, up to the cluster's limit (with 64 or 256 rows a CTA the LU of n = 1,000 takes 2-3%
-// longer in complex64, 1-6% in complex128). Per CTA: one row a thread and 16 columns a group as long as the registers
-// allow (groups of 8 at 256 rows: 2-6% longer LUs, twice the group ends), then fewer columns a group and more rows a
-// thread. Whole LUs, complex64 / complex128, when the choice was made (both sides are shorter now): n = 1,000 2.82 /
-// 3.18 ms, 4,977 16.7 / 22.1 ms; with two rows a thread of 128 for 256 rows 2.83 / 3.31 and 17.5 / 23.2 ms; above 512
-// rows, complex64, 16 columns and two rows a thread of 512 (spilling) 43.7 against 43.1 ms at n = 9,601.
+// longer in complex64, 1-6% in complex128). Per CTA: one row a thread and 16 columns a group up to 256 rows (groups of 8
+// there: 2-6% longer LUs, twice the group ends; two rows a thread of 128: 2.83 / 3.31 ms against 2.82 / 3.18 at n =
+// 1,000, 17.5 / 23.2 against 16.7 / 22.1 at 4,977, complex64 / complex128), then fewer columns a group and more rows a
+// thread. The kernels of 512 threads (above 256 rows a CTA in complex64, 512 in complex128) are held to 128 registers and
+// spill: 156 bytes a thread stored in <float, 16, 1>, 436 in <float, 8, 4>, 752 in <double, 8, 2>; above 512 rows,
+// complex64, 16 columns and two rows a thread of 512 take 43.7 ms against 43.1 at n = 9,601. (LU times of the tree that
+// the choices were made on; the panel's later changes shortened both sides of each.)
 int m25_panel_cluster(void *A, long lda, int n, int k0, int jb, int *ipiv, int single, int cl, int *err, cudaStream_t s)
 {
     const int rows = n - k0;
