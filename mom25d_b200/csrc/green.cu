@@ -369,7 +369,9 @@ __global__ void k_contour(double t1, double alpha, double K, double wid2, int m1
 // 88 us, with 4 blocks 100). Clusters of four do not fill every group of SMs: on 148 SMs 70 of them still do, 74 do not,
 // so the line is drawn at 64. Measured with 1 / 4 blocks: 1,500 points and 4, 8, 16 spectra, 64 radii 36.5 / 35.6,
 // 36.8 / 34.8, 38.9 / 36.7 us, 100 radii 36.8 / 37.8, 37.1 / 53.6, 38.9 / 56.5, 148 radii 36.5 / 53.3, 37.5 / 62.0,
-// 40.0 / 66.1; 6,000 points and 8 spectra, 64 radii 65.6 / 41.1, 100 66.0 / 63.8, 148 66.1 / 78.2.
+// 40.0 / 66.1; 6,000 points and 8 spectra, 64 radii 65.6 / 41.1, 100 66.0 / 63.8, 148 66.1 / 78.2. One block, too, up to
+// 512 points, two a thread: 40 radii, 16 spectra, 300 points 32.9 / 32.8 us (real contour 16.0 / 20.4), 512 32.5 / 32.8
+// (17.8 / 18.3), 600 34.9 / 33.2 (18.0 / 18.4), 800 36.0 / 32.8 (19.9 / 18.2).
 // RAW: the bare sum over real kr (hankel_real, mom25d_core.cpp:1430-1454): out[s, i] = sum_k J0(rho_i kr_k) W[s, k],
 // kr_ real f64[npts], no dk, no 1 / 2 pi.
 template <int NS, int HB, bool RAW = false>
@@ -692,7 +694,7 @@ static void hankel_launch(const double *kr, const double *dk, int npts, const do
         (void)cudaGetLastError();
     auto go = [&](auto nsm) {
         constexpr int NS = decltype(nsm)::value;
-        if (16 * (long)nr > 7 * (long)sms) k_hankel<NS, 1, RAW><<<nr, 256, 0, s>>>(kr, dk, npts, W, ns, rho, out, nr);
+        if (npts <= 512 || 16 * (long)nr > 7 * (long)sms) k_hankel<NS, 1, RAW><<<nr, 256, 0, s>>>(kr, dk, npts, W, ns, rho, out, nr);
         else k_hankel<NS, 4, RAW><<<dim3(nr, 4), 256, 0, s>>>(kr, dk, npts, W, ns, rho, out, nr);
     };
     if (ns <= 4) go(std::integral_constant<int, 4>());
